@@ -264,7 +264,7 @@ int pfxt_trace_counts_device(pfxt_trace* t, const pfxt_ray* rays, uint32_t count
                              void* stream) {
   return guarded([&]() {
     if (!t || (count && (!rays || !counts))) throw Invalid("null argument");
-    check(launch_counts(t->view, rays, count, any != 0, reinterpret_cast<uint2*>(counts), next_counter(*t),
+    check(launch_counts(t->view, rays, count, any != 0, reinterpret_cast<uint2*>(counts),
                         (cudaStream_t)stream),
           "counting kernel");
   });

@@ -22,6 +22,8 @@ cudaError_t prepare_any_queries();
 // scratch arrays on `device`, which must be current.
 cudaError_t noalloc_prepare(int device);
 cudaError_t launch_counts(const SceneView& s, const pfxt_ray* rays, uint32_t n, bool any, uint2* counts,
-                          uint32_t* counter, cudaStream_t stream);
+                          cudaStream_t stream);
+// The four-box nodes of `n` two-box nodes, by the same index.
+cudaError_t launch_collapse(const WideNode* wide, uint32_t n, QuadNode* quad, cudaStream_t stream);
 
 }  // namespace pfxt

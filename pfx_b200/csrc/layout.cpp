@@ -45,10 +45,57 @@ struct Builder {
   std::unordered_map<uint32_t, uint64_t> reach_of;
   uint64_t reach = 0;  // running maximum while one subtree is laid out
 
+  // The slot base of the subtree being laid out (0: the top level's own
+  // leaves), the base each pseudo-parent's subtree was laid out with, and
+  // which slots have their leaf's box.  Scene builds put a slot in one leaf;
+  // buffers that do not are walked with the two-box nodes alone (`unboxed`).
+  uint32_t base = 0;
+  std::unordered_map<uint32_t, uint32_t> base_of;
+  std::vector<uint8_t> boxed;
+  bool unboxed = false;
+  // Entries the four-box walk's stack needs (the buffers' own max_depth is the
+  // caller's word, and the two-box walk's): below the child laid out last as one
+  // entry, and below its own two children when it is an inner node; below each
+  // pseudo-parent's root as a node of its own.
+  struct Need {
+    uint32_t whole = 0, child[2] = {0, 0};
+    bool inner = false;
+  } need;
+  std::unordered_map<uint32_t, uint32_t> need_of;
+
+  // Of a node whose children need l and r: inside entry i of its four, the
+  // entries after i wait.
+  static uint32_t quad_need(const Need& l, const Need& r) {
+    uint32_t list[4], n = 0, most = 0;
+    for (const Need* c : {&l, &r}) {
+      if (c->inner) {
+        list[n++] = c->child[0];
+        list[n++] = c->child[1];
+      } else {
+        list[n++] = c->whole;
+      }
+    }
+    for (uint32_t i = 0; i < n; ++i) most = std::max(most, n - 1u - i + list[i]);
+    return most;
+  }
+
+  void box_leaf(const GpuNode& n) {
+    const uint64_t first = (uint64_t)base + n.first;
+    if (first + n.count > tri_count) return;  // refused by the reach check
+    for (uint64_t i = first; i < first + n.count; ++i) {
+      TravTri& t = out.tris[i];
+      if (boxed[i] && (memcmp(t.lo, n.lo, 12) != 0 || memcmp(t.hi, n.hi, 12) != 0)) unboxed = true;
+      memcpy(t.lo, n.lo, 12);
+      memcpy(t.hi, n.hi, 12);
+      boxed[i] = 1u;
+    }
+  }
+
   uint32_t leaf_ref(const GpuNode& n) {
     if (n.count == 0 || n.count > 16) throw Invalid("BVH leaf holds more than 16 triangles");
     if (n.first > LEAF_FIRST_MASK) throw Invalid("BVH leaf offset exceeds the traversal encoding");
     reach = std::max<uint64_t>(reach, (uint64_t)n.first + n.count);
+    box_leaf(n);
     return REF_LEAF | ((n.count - 1u) << LEAF_FIRST_BITS) | n.first;
   }
 
@@ -75,11 +122,19 @@ struct Builder {
       r.inv[2][3] = bits2f(m.pad[1]);
     }
     if (n.first >= node_count) throw Invalid("instance root out of range");
+    memcpy(r.lo, n.lo, 12);
+    memcpy(r.hi, n.hi, 12);
     uint64_t outer = reach;
+    uint32_t outer_base = base;
     reach = 0;
+    base = r.base;
     r.root = pseudo(n.first);
     uint64_t inner = reach_of[r.root];
+    if (base_of[r.root] != r.base) unboxed = true;
+    need = Need{};
+    need.whole = 1u + need_of[r.root];  // the sentinel that ends the instance
     reach = outer;
+    base = outer_base;
     if ((uint64_t)r.base + inner > tri_count) throw Invalid("an instance leaf reaches past the triangles");
     uint32_t index = (uint32_t)out.insts.size();
     if (index >= (1u << 30)) throw Invalid("too many instances");
@@ -92,6 +147,7 @@ struct Builder {
     const GpuNode& n = nodes[i];
     if (n.pad[0] == INSTANCE_LEAF) return inst_ref(n);
     if (n.count == 0) return wide_of(i);
+    need = Need{};
     return leaf_ref(n);
   }
 
@@ -101,6 +157,7 @@ struct Builder {
     uint32_t w = (uint32_t)out.wide.size();
     out.wide.push_back(WideNode{});
     pseudo_of[root] = w;
+    base_of[w] = base;
     uint64_t outer = reach;
     reach = 0;
     WideNode node{};
@@ -108,6 +165,7 @@ struct Builder {
     node.child[0] = child_ref(root);
     node.child[1] = REF_NONE;
     out.wide[w] = node;
+    need_of[w] = need.whole;
     reach_of[w] = reach;
     reach = outer;
     return w;
@@ -124,7 +182,13 @@ struct Builder {
     set_box(node, 0, nodes[left]);
     set_box(node, 1, nodes[right]);
     node.child[0] = child_ref(left);
+    const Need l = need;
     node.child[1] = child_ref(right);
+    const Need r = need;
+    need.whole = quad_need(l, r);
+    need.child[0] = l.whole;
+    need.child[1] = r.whole;
+    need.inner = true;
     out.wide[w] = node;
     return w;
   }
@@ -140,27 +204,34 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
   builder.surface_count = b.surfaces_bytes / sizeof(GpuSurface);
   builder.tri_count = b.triangles_bytes / sizeof(GpuTriangle);
   if (b.triangle_count != builder.tri_count) throw Invalid("triangle count does not match the triangle buffer");
+  builder.out.tris.resize(builder.tri_count);
+  builder.boxed.assign(builder.tri_count, 0u);
   if (builder.node_count > 0 && b.triangle_count > 0) {
     builder.out.wide.reserve(builder.node_count / 2 + 16);
     builder.out.root = builder.pseudo(0);
     // the top level itself: world leaves (base 0) must stay inside the triangles
     if (builder.reach_of[builder.out.root] > builder.tri_count)
       throw Invalid("a BVH leaf reaches past the triangles");
+    if (builder.need_of[builder.out.root] > QUAD_STACK) builder.unboxed = true;
   }
   // The box test needs no range check on its quotients when every box
   // coordinate is 0 or of magnitude in [2^-70, 2^79] (traverse.cuh,
-  // BOUNDED_TINY and BOUNDED_COORD); NaN coordinates fail this too.
-  builder.out.small = true;
+  // BOUNDED_TINY and BOUNDED_COORD); NaN coordinates fail this too.  The
+  // four-box walk also picks the planes that a ray enters through by its
+  // direction's signs, which asks for lo <= hi, and leaves whose triangles
+  // know their box, and a stack that fits QUAD_STACK entries.
+  builder.out.small = !builder.unboxed;
   for (const WideNode& w : builder.out.wide) {
     const float* f = &w.b0[0];
     for (int k = 0; k < 12; ++k) {
       float a = std::fabs(f[k]);
       if (!(a == 0.0f || (a >= 0x1p-70f && a <= 0x1p+79f))) builder.out.small = false;
     }
+    for (int k = 0; k < 3; ++k)
+      if (!(f[k] <= f[3 + k]) || !(f[6 + k] <= f[9 + k])) builder.out.small = false;
   }
   const GpuTriangle* tris = (const GpuTriangle*)b.triangles;
   size_t count = b.triangles_bytes / sizeof(GpuTriangle);
-  builder.out.tris.resize(count);
   for (size_t i = 0; i < count; ++i) {
     const GpuTriangle& t = tris[i];
     TravTri& o = builder.out.tris[i];
@@ -169,9 +240,6 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
       o.e1[k] = t.b[k] - t.a[k];  // tri_hit: e1 = tri.b.xyz - tri.a.xyz
       o.e2[k] = t.c[k] - t.a[k];  // e2 = tri.c.xyz - tri.a.xyz
     }
-    o.a[3] = 0.0f;
-    o.e1[3] = 0.0f;
-    o.e2[3] = 0.0f;
   }
   return std::move(builder.out);
 }

@@ -7,10 +7,10 @@
 //    record.rs:18-27 Hot 128 B).  They are the drop-in seam: a host that already
 //    packs SceneBuffers hands these bytes over unchanged;
 //  * the B200 traversal layout derived from them on upload: 64-byte two-box
-//    nodes (both children's fp32 boxes in the parent, one 4 x 16 B fetch per
-//    pair of box tests), 48-byte triangles (vertex a and the two edges,
-//    precomputed with the same fp32 subtraction the reference does per test) and
-//    64-byte instance records.
+//    nodes (both children's fp32 boxes in the parent), 128-byte four-box nodes
+//    collapsed from them, 64-byte triangles (vertex a and the two edges,
+//    precomputed with the same fp32 subtraction the reference does per test,
+//    and the leaf's box) and 96-byte instance records.
 #pragma once
 #include <stdint.h>
 
@@ -94,12 +94,27 @@ struct alignas(16) WideNode {
 };
 static_assert(sizeof(WideNode) == 64, "WideNode");
 
-struct alignas(16) TravTri {
-  float a[4];   // a.xyz
-  float e1[4];  // b - a
-  float e2[4];  // c - a
+// Four-box node of the closest- and any-hit walks: the grandchildren of an
+// inner node (or a child itself where it is a leaf), in the reference's
+// left-first order: one 32-byte sector of planes an axis and one with the
+// references.  Unused children hold the empty box (+inf, -inf).
+struct alignas(128) QuadNode {
+  struct {
+    float lo[4], hi[4];
+  } axis[3];
+  uint32_t child[4];
+  uint32_t pad[4];
 };
-static_assert(sizeof(TravTri) == 48, "TravTri");
+static_assert(sizeof(QuadNode) == 128, "QuadNode");
+
+// A triangle (vertex a, the two edges) and the exact box of the leaf that
+// holds it; the first three 16-byte words are all that the triangle test reads.
+struct alignas(64) TravTri {
+  float a[3], e1[3], e2[3];  // a, b - a, c - a
+  float lo[3], hi[3];        // the leaf's box
+  float pad;
+};
+static_assert(sizeof(TravTri) == 64, "TravTri");
 
 struct alignas(16) InstRec {
   float inv[3][4];     // inverse rows (world -> object), levels.rs:457-467
@@ -109,11 +124,17 @@ struct alignas(16) InstRec {
   uint32_t word;       // instance word
   float inv_det;       // inverse determinant (object-space det sign/scale)
   uint32_t transformed;  // 0: the ray stays in world space (the world group)
-  uint32_t pad[2];
+  float lo[3], hi[3];  // the instance leaf's exact world box
 };
-static_assert(sizeof(InstRec) == 80, "InstRec");
+static_assert(sizeof(InstRec) == 96, "InstRec");
 
 // Stack bound of the reference traversal (trace.wgsl:1003, 64 entries).
 constexpr uint32_t REF_STACK = 64u;
+// Stack entries of the four-box walk.  It waits on up to three siblings a node
+// where the reference waits on one per level; layout.cpp works out what a
+// scene needs, and one that needs more takes the two-box walk.  (The 1.19 M
+// triangle room needs under 40; 128 entries made the local memory of every
+// resident thread 1 KB.)
+constexpr uint32_t QUAD_STACK = 64u;
 
 }  // namespace pfxt

@@ -453,13 +453,14 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
   uint32_t* counter = P.w.counters + (ANY ? 16 : 4);
   __shared__ uint32_t short_ref[SHORT > 0 ? SHORT * THREADS : 1];
   __shared__ float short_near[SHORT > 0 ? SHORT * THREADS : 1];
-  LaneStack<SHORT> st;
+  LaneStack<SHORT, (int)QUAD_STACK> st;
   if constexpr (SHORT > 0) {
     st.sh_ref = short_ref + threadIdx.x;
     st.sh_near = short_near + threadIdx.x;
     st.lanes = THREADS;
   }
-  Walker<ANY, false, TRACE_BOX, TRACE_SPEC> w;
+  QuadWalker<ANY> w;
+  w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0, item = 0;
   bool have = false, retired = false;
@@ -485,25 +486,23 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
       }
     }
     if (__all_sync(FULL, retired)) break;
-    if (have) {
-      w.inner_phase(P.s, st, [&](v3& o, v3& d) {
-        float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
-        float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
-        o = mk3(a.x, a.y, a.z);
-        d = mk3(b.x, b.y, b.z);
-      });
-      if (w.leaf_ready()) w.leaf_phase(P.s, st);
-      if (!w.leaf_ready()) {
-        if (w.retry) {
-          (ANY ? P.w.retry : P.w.eretry)[atomicAdd(P.w.counters + (ANY ? 14 : 13), 1u)] = item;
-        } else if (ANY) {
-          reinterpret_cast<float*>(P.w.sh_d + item)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
-        } else {
-          P.w.hit[item] = make_float4(w.hit.t, __uint_as_float(w.hit.slot), __uint_as_float(w.hit.record), w.hit.u);
-          P.w.hit_v[item] = w.hit.v;
-        }
-        have = false;
+    w.inner_phase(P.s, st, [&](v3& o, v3& d) {
+      float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
+      float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
+      o = mk3(a.x, a.y, a.z);
+      d = mk3(b.x, b.y, b.z);
+    });
+    if (w.leaf_ready()) w.leaf_phase(P.s, st);
+    if (have && w.finished()) {
+      if (w.hit.hit == QuadWalker<ANY>::RETRY) {
+        (ANY ? P.w.retry : P.w.eretry)[atomicAdd(P.w.counters + (ANY ? 14 : 13), 1u)] = item;
+      } else if (ANY) {
+        reinterpret_cast<float*>(P.w.sh_d + item)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
+      } else {
+        P.w.hit[item] = make_float4(w.hit.t, __uint_as_float(w.hit.slot), __uint_as_float(w.record(P.s)), w.hit.u);
+        P.w.hit_v[item] = w.hit.v;
       }
+      have = false;
     }
   }
 }
@@ -519,7 +518,7 @@ __global__ void __launch_bounds__(128) k_trace_queue_retry(const __grid_constant
     const uint32_t item = (ANY ? P.w.retry : P.w.eretry)[k];
     float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
     float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
-    LaneStack<0> st;
+    RefStack st;
     Walker<ANY, false, BOX_IEEE> w;
     w.start(P.s, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), ANY ? a.w : 1e20f);
     w.run(P.s, st, [&](v3& o, v3& d) {

@@ -88,6 +88,7 @@ struct pfxt_trace {
   uint32_t projection = 0;
   // traversal layout
   pfxt::WideNode* d_wide = nullptr;
+  pfxt::QuadNode* d_quad = nullptr;
   pfxt::TravTri* d_tris = nullptr;
   pfxt::InstRec* d_insts = nullptr;
   pfxt::SceneView view{};

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "cache.h"
+#include "kernels.h"
 #include "tracer.h"
 
 namespace pfxt {
@@ -41,6 +42,16 @@ void* dev_copy(pfxt_trace& t, const void* host, size_t bytes, const char* what) 
 template <typename T>
 T* dev_alloc(pfxt_trace& t, size_t count, const char* what) {
   return static_cast<T*>(dev_copy(t, nullptr, count * sizeof(T), what));
+}
+
+// The four-box nodes of `n` two-box nodes on the device.
+QuadNode* dev_quads(pfxt_trace& t, const WideNode* wide, size_t n) {
+  QuadNode* d = nullptr;
+  check(cudaMalloc(&d, std::max<size_t>(n, 1) * sizeof(QuadNode)), "nodes");
+  t.owned.push_back(d);
+  check(launch_collapse(wide, (uint32_t)n, d, t.stream), "nodes");
+  check(cudaStreamSynchronize(t.stream), "nodes");
+  return d;
 }
 
 bool finite3(const float* p) { return std::isfinite(p[0]) && std::isfinite(p[1]) && std::isfinite(p[2]); }
@@ -73,7 +84,9 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
   t.d_tris = static_cast<TravTri*>(dev_copy(t, layout.tris.data(), layout.tris.size() * sizeof(TravTri), "triangles"));
   t.d_insts =
       static_cast<InstRec*>(dev_copy(t, layout.insts.data(), layout.insts.size() * sizeof(InstRec), "instances"));
+  t.d_quad = dev_quads(t, t.d_wide, layout.wide.size());
   t.view.wide = t.d_wide;
+  t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;
   t.view.insts = t.d_insts;
   t.view.root = layout.root;
@@ -306,17 +319,18 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b) {
   check(cudaStreamSynchronize(t.stream), "move instances");
   // New traversal buffers first, so that a failed allocation leaves the trace as it was.
   size_t kept = t.owned.size();
-  void* fresh[3] = {nullptr, nullptr, nullptr};
+  void* fresh[4] = {nullptr, nullptr, nullptr, nullptr};
   try {
     fresh[0] = dev_copy(t, layout.wide.data(), layout.wide.size() * sizeof(WideNode), "nodes");
     fresh[1] = dev_copy(t, layout.tris.data(), layout.tris.size() * sizeof(TravTri), "triangles");
     fresh[2] = dev_copy(t, layout.insts.data(), layout.insts.size() * sizeof(InstRec), "instances");
+    fresh[3] = dev_quads(t, static_cast<const WideNode*>(fresh[0]), layout.wide.size());
   } catch (...) {
     for (size_t i = kept; i < t.owned.size(); ++i) cudaFree(t.owned[i]);
     t.owned.resize(kept);
     throw;
   }
-  void* stale[3] = {t.d_wide, t.d_tris, t.d_insts};
+  void* stale[4] = {t.d_wide, t.d_tris, t.d_insts, t.d_quad};
   for (void* p : stale) {
     auto it = std::find(t.owned.begin(), t.owned.end(), p);
     if (it != t.owned.end()) {
@@ -327,7 +341,9 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b) {
   t.d_wide = static_cast<WideNode*>(fresh[0]);
   t.d_tris = static_cast<TravTri*>(fresh[1]);
   t.d_insts = static_cast<InstRec*>(fresh[2]);
+  t.d_quad = static_cast<QuadNode*>(fresh[3]);
   t.view.wide = t.d_wide;
+  t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;
   t.view.insts = t.d_insts;
   t.view.root = layout.root;
@@ -470,16 +486,26 @@ pfxt_tuning trace_get_tuning(const pfxt_trace& t) {
 }
 
 // FNV-1a style mixing of 8-byte words (and the bytes left over), continuing
-// from `h`: a fingerprint, not a format.
+// from `h`: a fingerprint, not a format.  Four chains side by side, as one is
+// bound by the multiplier's latency.
 uint64_t fnv(uint64_t h, const void* data, size_t bytes) {
   const unsigned char* p = static_cast<const unsigned char*>(data);
-  size_t words = bytes / 8;
-  for (size_t i = 0; i < words; ++i) {
+  size_t words = bytes / 8, i = 0;
+  uint64_t lane[4] = {h, ~h, h + 1u, ~h - 1u};
+  for (; i + 4 <= words; i += 4)
+    for (size_t k = 0; k < 4; ++k) {
+      uint64_t w;
+      memcpy(&w, p + 8 * (i + k), 8);
+      lane[k] = (lane[k] ^ w) * 0x100000001b3ull;
+    }
+  if (i)
+    for (uint64_t l : lane) h = (h ^ l) * 0x100000001b3ull;
+  for (; i < words; ++i) {
     uint64_t w;
     memcpy(&w, p + 8 * i, 8);
     h = (h ^ w) * 0x100000001b3ull;
   }
-  for (size_t i = 8 * words; i < bytes; ++i) h = (h ^ p[i]) * 0x100000001b3ull;
+  for (i = 8 * words; i < bytes; ++i) h = (h ^ p[i]) * 0x100000001b3ull;
   return h;
 }
 

@@ -33,20 +33,18 @@ __device__ __forceinline__ void load_ray(const pfxt_ray* __restrict__ rays, uint
 
 // The output word that marks a ray the first walk handed over to the IEEE
 // walk (closest hit: the `hit` field; any hit: the flag).
-constexpr uint32_t RETRY = 2u;
+constexpr uint32_t RETRY = QuadWalker<true>::RETRY;
 
-// MODE 0: closest hit -> pfxt_hit; MODE 1: any hit -> u32 flag;
-// MODE 2/3: work counters of closest / any hit -> uint2.  Modes 0 and 1 walk
-// bounded rays only (no call in the walk loop) and mark the others RETRY for
-// k_trace_retry; the counting modes walk every ray.
+// MODE 0: closest hit -> pfxt_hit; MODE 1: any hit -> u32 flag.  Rays that the
+// four-box walk cannot take are marked RETRY for k_trace_retry.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, TRACE_WARPS_PER_SM * 32 / kThreads) k_trace(SceneView s, const pfxt_ray* __restrict__ rays, uint32_t n,
                                                     void* __restrict__ out, uint32_t* __restrict__ counter) {
-  constexpr bool ANY = (MODE == 1 || MODE == 3);
-  constexpr bool COUNT = (MODE >= 2);
+  constexpr bool ANY = MODE == 1;
   constexpr unsigned FULL = 0xffffffffu;
-  LaneStack<0> st;  // local memory: a shared-memory top measured slower (more registers, fewer warps)
-  Walker<ANY, COUNT, COUNT ? BOX_EITHER : TRACE_BOX, !COUNT && TRACE_SPEC> w;
+  QuadStack st;
+  QuadWalker<ANY> w;
+  w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0;
   bool have = false, retired = false;
@@ -72,23 +70,18 @@ __global__ void __launch_bounds__(kThreads, TRACE_WARPS_PER_SM * 32 / kThreads) 
       }
     }
     if (__all_sync(FULL, retired)) break;
-    if (have) {
-      w.inner_phase(s, st, [&](v3& o, v3& d) {
-        float tmax;
-        load_ray(rays, idx, o, d, tmax);
-      });
-      if (w.leaf_ready()) w.leaf_phase(s, st);
-      if (!w.leaf_ready()) {
-        if (MODE == 0) {
-          reinterpret_cast<uint4*>(out)[idx] =
-              make_uint4(__float_as_uint(w.hit.t), w.hit.slot, w.hit.record, w.retry ? RETRY : w.hit.hit);
-        } else if (MODE == 1) {
-          reinterpret_cast<uint32_t*>(out)[idx] = w.retry ? RETRY : w.hit.hit;
-        } else {
-          reinterpret_cast<uint2*>(out)[idx] = make_uint2(w.counts.boxes, w.counts.tris);
-        }
-        have = false;
-      }
+    w.inner_phase(s, st, [&](v3& o, v3& d) {
+      float tmax;
+      load_ray(rays, idx, o, d, tmax);
+    });
+    if (w.leaf_ready()) w.leaf_phase(s, st);
+    if (have && w.finished()) {
+      if (MODE == 0)
+        reinterpret_cast<uint4*>(out)[idx] =
+            make_uint4(__float_as_uint(w.hit.t), w.hit.slot, w.record(s), w.hit.hit);
+      else
+        reinterpret_cast<uint32_t*>(out)[idx] = w.hit.hit;
+      have = false;
     }
   }
 }
@@ -103,7 +96,7 @@ __global__ void __launch_bounds__(kThreads) k_trace_retry(SceneView s, const pfx
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     uint32_t marker = MODE == 0 ? reinterpret_cast<const uint4*>(out)[i].w : reinterpret_cast<const uint32_t*>(out)[i];
     if (marker != RETRY) continue;
-    LaneStack<0> st;
+    RefStack st;
     Walker<ANY, false, BOX_IEEE> w;
     v3 o, d;
     float tmax;
@@ -118,6 +111,67 @@ __global__ void __launch_bounds__(kThreads) k_trace_retry(SceneView s, const pfx
     else
       reinterpret_cast<uint32_t*>(out)[i] = w.hit.hit;
   }
+}
+
+// Box and triangle tests of every ray as the reference counts them, one ray a
+// thread on the two-box nodes (a measurement, not a hot path).
+template <bool ANY>
+__global__ void __launch_bounds__(kThreads) k_trace_counts(SceneView s, const pfxt_ray* __restrict__ rays, uint32_t n,
+                                                           uint2* __restrict__ out) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    RefStack st;
+    Walker<ANY, true, BOX_EITHER> w;
+    v3 o, d;
+    float tmax;
+    load_ray(rays, i, o, d, tmax);
+    w.start(s, o, d, tmax);
+    w.run(s, st, [&](v3& wo, v3& wd) {
+      wo = o;
+      wd = d;
+    });
+    out[i] = make_uint2(w.counts.boxes, w.counts.tris);
+  }
+}
+
+// The four-box node of every two-box node: its grandchildren, or a child
+// itself where that is a leaf; for a pseudo-parent (one child, a subtree's
+// root) the root's.  Nodes that only another node's expansion reaches are
+// written too and never read: an index per two-box node needs no numbering
+// pass, and the lines the walk does not touch cost no cache.
+__global__ void __launch_bounds__(kThreads) k_collapse(const WideNode* __restrict__ wide, uint32_t n,
+                                                       QuadNode* __restrict__ quad) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  QuadNode q;
+  for (int k = 0; k < 4; ++k) {
+    for (int x = 0; x < 3; ++x) {
+      q.axis[x].lo[k] = INFINITY;
+      q.axis[x].hi[k] = -INFINITY;
+    }
+    q.child[k] = REF_NONE;
+    q.pad[k] = 0u;
+  }
+  int count = 0;
+  auto add = [&](const WideNode& w, int c) {
+    const float* f = &w.b0[0] + 6 * c;
+    for (int x = 0; x < 3; ++x) {
+      q.axis[x].lo[count] = f[x];
+      q.axis[x].hi[count] = f[3 + x];
+    }
+    q.child[count++] = w.child[c];
+  };
+  const uint32_t top = wide[i].child[1] == REF_NONE && !(wide[i].child[0] & REF_LEAF) ? wide[i].child[0] : i;
+  for (int c = 0; c < 2; ++c) {
+    const uint32_t child = wide[top].child[c];
+    if (child == REF_NONE) continue;
+    if (child & REF_LEAF) {
+      add(wide[top], c);
+    } else {
+      add(wide[child], 0);
+      if (wide[child].child[1] != REF_NONE) add(wide[child], 1);
+    }
+  }
+  quad[i] = q;
 }
 
 // Narrow 32-bit flags to bytes (separate input and output regions).
@@ -158,10 +212,7 @@ cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* o
   uint32_t blocks = (uint32_t)persistent_blocks<MODE>();
   if (need < blocks) blocks = need;
   k_trace<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter);
-  if constexpr (MODE < 2) {
-    uint32_t scan = (n + kThreads - 1) / kThreads, most = (uint32_t)persistent_blocks<MODE>();
-    k_trace_retry<MODE><<<scan < most ? scan : most, kThreads, 0, stream>>>(s, rays, n, out);
-  }
+  k_trace_retry<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out);
   return cudaGetLastError();
 }
 
@@ -178,8 +229,20 @@ cudaError_t launch_any(const SceneView& s, const pfxt_ray* rays, uint32_t n, uin
 }
 
 cudaError_t launch_counts(const SceneView& s, const pfxt_ray* rays, uint32_t n, bool any, uint2* counts,
-                          uint32_t* counter, cudaStream_t stream) {
-  return any ? launch<3>(s, rays, n, counts, counter, stream) : launch<2>(s, rays, n, counts, counter, stream);
+                          cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  const uint32_t blocks = (n + kThreads - 1) / kThreads;
+  if (any)
+    k_trace_counts<true><<<blocks, kThreads, 0, stream>>>(s, rays, n, counts);
+  else
+    k_trace_counts<false><<<blocks, kThreads, 0, stream>>>(s, rays, n, counts);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_collapse(const WideNode* wide, uint32_t n, QuadNode* quad, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  k_collapse<<<(n + kThreads - 1) / kThreads, kThreads, 0, stream>>>(wide, n, quad);
+  return cudaGetLastError();
 }
 
 cudaError_t prepare_any_queries() {

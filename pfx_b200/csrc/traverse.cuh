@@ -12,13 +12,25 @@
 // motion and analytic shapes are outside this library's scope; the scenes it
 // accepts have none.
 //
+// Two walks.
+//  * QuadWalker, the one the batch and queue kernels run: four-box nodes
+//    (QuadNode) tested with quotients that are a rounding or two off and a
+//    comparison widened by more than that, so it may open a box that the
+//    reference skips but never skips one that the reference opens; where a
+//    triangle would be accepted, its leaf's own box is tested as the reference
+//    tests it, and the leaf is dropped if that fails.  Rays it cannot take are
+//    marked for retry.
+//  * Walker, on the two-box nodes with the reference's own box tests: the
+//    work-counting kernels, the retry kernels (IEEE division throughout) and
+//    queries inside shading code.
+//
 // The per-ray stack holds (entry, near) pairs.  `near` is the entry distance
 // of the child box computed when its parent was opened; box_hit(node, hit.t)
 // at pop time is exactly "geometry passes && near <= hit.t", so re-checking
 // near against the current hit distance on pop reproduces the reference's
-// pruning.  The stack never holds more entries than the reference's 64-entry
-// stack holds at the same point; scenes that would overflow that stack are
-// refused when they are created.
+// pruning.  Walker's stack never holds more entries than the reference's
+// 64-entry stack holds at the same point; scenes that would overflow that
+// stack are refused when they are created.
 //
 // Work accounting (COUNT): the reference tests a node's box when it pops the
 // node, and it pushes both children of every inner node it opens.  The
@@ -35,10 +47,12 @@ constexpr uint32_t STACK_SENTINEL = 0xfffffffeu;
 
 struct SceneView {
   const WideNode* __restrict__ wide;
+  const QuadNode* __restrict__ quad;  // by the index of the two-box node it stands for
   const TravTri* __restrict__ tris;
   const InstRec* __restrict__ insts;
   uint32_t root;
-  uint32_t small;  // 1 when every box coordinate is 0 or in [BOUNDED_TINY, BOUNDED_COORD] in magnitude
+  uint32_t small;  // 1 when every box coordinate is 0 or in [BOUNDED_TINY, BOUNDED_COORD] in magnitude,
+                   // lo <= hi, and every leaf's triangles hold its box
 };
 
 struct TraceHit {
@@ -202,35 +216,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
-// A bounded ray whose direction has no degenerate axis, paired the way a
-// child box's six coordinates lie in a node, (lx, ly), (lz, hx), (hy, hz):
-// origins (ox, oy), (oz, ox), (oy, oz), reciprocals and negated directions
-// likewise.
-struct PRay {
-  f32x2 o[3], r[3], nd[3];
-};
-__device__ __forceinline__ PRay make_pray(const TRay& t) {
-  PRay p;
-  p.o[0] = pair(t.o.x, t.o.y);
-  p.o[1] = pair(t.o.z, t.o.x);
-  p.o[2] = pair(t.o.y, t.o.z);
-  p.r[0] = pair(t.r.x, t.r.y);
-  p.r[1] = pair(t.r.z, t.r.x);
-  p.r[2] = pair(t.r.y, t.r.z);
-  p.nd[0] = pair(-t.d.x, -t.d.y);
-  p.nd[1] = pair(-t.d.z, -t.d.x);
-  p.nd[2] = pair(-t.d.y, -t.d.z);
-  return p;
-}
-__device__ __forceinline__ bool packable(const TRay& t) {
-  return t.bounded && fabsf(t.d.x) >= 1e-12f && fabsf(t.d.y) >= 1e-12f && fabsf(t.d.z) >= 1e-12f;
-}
-
-// Markstein quotients of a pair: (x0/d0, x1/d1) correctly rounded, as quotient().
-__device__ __forceinline__ f32x2 quotient2(f32x2 x, f32x2 nd, f32x2 r) {
-  f32x2 q = mul2(x, r);
-  f32x2 e = fma2(q, nd, x);  // q * (-d) + x = fma(-q, d, x) exactly
-  return fma2(e, r, q);
+// 1/x to within an ulp (the hardware's approximation), for the loose box test.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 
 // The sm_100 three-input minimum and maximum: the same value as two two-input
@@ -246,56 +236,13 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
   return r;
 }
 
-// box_geometry_bounded for a ray with no degenerate axis, the box given as
-// the three coordinate pairs of its node: (lx, ly), (lz, hx), (hy, hz).
-__device__ __forceinline__ bool box_geometry_paired(f32x2 b0, f32x2 b1, f32x2 b2, const PRay& p, float& near) {
-  float lx, ly, lz, hx, hy, hz;
-  unpair(quotient2(sub2(b0, p.o[0]), p.nd[0], p.r[0]), lx, ly);
-  unpair(quotient2(sub2(b1, p.o[1]), p.nd[1], p.r[1]), lz, hx);
-  unpair(quotient2(sub2(b2, p.o[2]), p.nd[2], p.r[2]), hy, hz);
-  // max(0, entries) and min(exits), as box_geometry_bounded's chains
-  float n = fmaxf(max3f(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz)), 0.0f);
-  float f = min3f(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz));
-  near = n;
-  return !(n > f);
-}
-
-// How a walk tests boxes.
+// How Walker tests boxes.
 //  BOX_EITHER:  bounded rays with the Markstein quotients, other rays with the
 //               out-of-line IEEE test (one walk for every ray; the call costs
-//               the walk loop spills, so only the counting variant uses it);
-//  BOX_BOUNDED: Markstein quotients only; a ray that is not bounded (in world
-//               space or in an instance's space) stops at once with `retry`
-//               set, and a second kernel walks it again from the start with
-//               BOX_IEEE, so the walk loop has no call;
-//  BOX_IEEE:    IEEE division throughout, inline;
-//  BOX_PAIRED:  BOX_BOUNDED with the quotients in paired instructions; a ray
-//               with a degenerate axis is handed over like an unbounded one.
-// All four give the same bits for every box they test.
-constexpr int BOX_EITHER = 0, BOX_BOUNDED = 1, BOX_IEEE = 2, BOX_PAIRED = 3;
-// The flavour of the batch and queue traversal kernels (their retry kernels walk with BOX_IEEE) and
-// whether they set leaves aside (Walker's SPEC).  On the 4K room's pass mix (closest hit, 2^22 rays):
-// bounded 1023 Mrays/s, paired 1151, bounded with leaves set aside 1258, paired with leaves set aside
-// 1551; the plain 4K pass 133.3, 125.4, 105.0 and 95.2 ms.
-#ifndef TRACE_BOX
-#define TRACE_BOX BOX_PAIRED
-#endif
-#ifndef TRACE_SPEC
-#define TRACE_SPEC true
-#endif
-// Whether any-hit walks open the nearer child first (their result does not depend on the order).
-// Measured on the plain 4K pass: 94.6 ms nearer first against 92.4 ms left first.
-#ifndef TRACE_ANY_NEAR
-#define TRACE_ANY_NEAR false
-#endif
-// Whether a leaf set aside has its triangles prefetched: 0 no, 1 into L1 (prefetch.global.L1 per
-// line), 2 into L2 by one bulk prefetch (cp.async.bulk.prefetch.L2, the TMA unit).  Measured on the
-// pass mix (closest hit, 2^22 rays) and the plain 4K pass: none 1550 Mrays/s and 91.4 ms, L1 1470 and
-// 100.6 ms, L2 bulk 1489 and 94.5 ms.  The scene's nodes and triangles mostly sit in L2 already, and
-// the extra instructions cost more than the latency they hide.
-#ifndef TRACE_LEAF_PREFETCH
-#define TRACE_LEAF_PREFETCH 0
-#endif
+//               the walk loop spills);
+//  BOX_IEEE:    IEEE division throughout, inline.
+// Both give the same bits for every box they test.
+constexpr int BOX_EITHER = 0, BOX_IEEE = 2;
 
 template <int BOX>
 __device__ __forceinline__ bool box_test(float lx, float ly, float lz, float hx, float hy, float hz, const TRay& ray,
@@ -314,26 +261,20 @@ __device__ __forceinline__ v3 to_object(const float4& r0, const float4& r1, cons
   return o;
 }
 
-// The traversal stack of one lane.  With SHORT > 0 its first SHORT entries
-// live in shared memory, one column per lane (entry k of lane t at word
-// k * lanes + t, so a warp's accesses fall in distinct banks), and the rest
-// in local memory; with SHORT == 0 all of it is local.  Only where entries
-// are kept differs: the walk pushes and pops exactly the same entries.
-constexpr int SHORT_STACK = 16;
-
-// Resident warps per SM the traversal kernels are compiled for: it sets their
-// register budget.  32 warps (64 registers, a few bytes of spill) measured
-// faster than 24 (72 registers) and 36 (56 registers, more spills).
-#ifndef TRACE_WARPS_PER_SM
-#define TRACE_WARPS_PER_SM 32
-#endif
-
-template <int SHORT>
+// The traversal stack of one lane: (ref, near bits) pairs, one 8-byte store
+// per push and one 8-byte load per pop (measured 1037 against 1011 Mrays/s
+// with two 4-byte arrays).  With SHORT > 0 the first SHORT entries live in
+// shared memory, one column per lane (entry k of lane t at word k * lanes + t,
+// so a warp's accesses fall in distinct banks), and the rest in local memory;
+// with SHORT == 0 all of it is local.  Only where entries are kept differs:
+// the walk pushes and pops exactly the same entries.
+template <int SHORT, int DEPTH>
 struct LaneStack {
+  static constexpr int CAPACITY = DEPTH;
   uint32_t* sh_ref;
   float* sh_near;
   uint32_t lanes;
-  uint2 entry[REF_STACK - SHORT];  // (ref, near bits) pairs past the shared-memory top
+  uint2 entry[DEPTH - SHORT];  // past the shared-memory top
   __device__ __forceinline__ void put(int k, uint32_t r, float n) {
     if (k < SHORT) {
       sh_ref[k * lanes] = r;
@@ -353,12 +294,10 @@ struct LaneStack {
     }
   }
 };
-
-// Entries as (ref, near bits) pairs: one 8-byte store per push and one 8-byte
-// load per pop (measured 1037 against 1011 Mrays/s with two 4-byte arrays).
-template <>
-struct LaneStack<0> {
-  uint2 entry[REF_STACK];
+template <int DEPTH>
+struct LaneStack<0, DEPTH> {
+  static constexpr int CAPACITY = DEPTH;
+  uint2 entry[DEPTH];
   __device__ __forceinline__ void put(int k, uint32_t r, float n) { entry[k] = make_uint2(r, __float_as_uint(n)); }
   __device__ __forceinline__ void get(int k, uint32_t& r, float& n) const {
     uint2 e = entry[k];
@@ -366,36 +305,63 @@ struct LaneStack<0> {
     n = __uint_as_float(e.y);
   }
 };
+using RefStack = LaneStack<0, (int)REF_STACK>;
+using QuadStack = LaneStack<0, (int)QUAD_STACK>;
 
-// One query's traversal state; the stack is the caller's.
-// SPEC: a lane that reaches a leaf while other lanes of its warp still walk
-// inner nodes sets the leaf aside (`held`) and walks on, so that the warp's
-// leaf tests run with more lanes at once (Aila and Laine, "Understanding the
-// efficiency of ray traversal on GPUs", 2009).  It tests the leaves the
-// reference tests, in the reference's order, with the same hit distance at
-// each: the held leaf is the next one in the reference's order and is tested
-// before any other; everything walked past it was decided against the hit
-// distance from before its test, which is not smaller than the reference's, so
-// the walk only keeps more entries; and each of those is checked again
-// against the current distance before it is opened or tested (a node's entry
-// distance is at least its ancestors' in the same space, as a box holds its
-// children's).  A held leaf is tested before the walk enters or leaves an
-// instance, so it is tested in its own space.  Entries are right siblings of
-// the current path, as in the reference, so the stack is no deeper.
-template <bool ANY, bool COUNT, int BOX = BOX_EITHER, bool SPEC = false>
+// Resident warps per SM the traversal kernels are compiled for: it sets their
+// register budget.
+#ifndef TRACE_WARPS_PER_SM
+#define TRACE_WARPS_PER_SM 32
+#endif
+
+// One 32-byte sector in one load (sm_100's 256-bit loads), as pairs.
+__device__ __forceinline__ void load32(const void* p, f32x2 (&q)[4]) {
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(q[0]), "=l"(q[1]), "=l"(q[2]), "=l"(q[3]) : "l"(p));
+}
+
+// The nine numbers of a triangle that its test reads.
+__device__ __forceinline__ void load_tri(const TravTri* t, v3& a, v3& e1, v3& e2) {
+  f32x2 q[4];
+  load32(t, q);
+  unpair(q[0], a.x, a.y);
+  unpair(q[1], a.z, e1.x);
+  unpair(q[2], e1.y, e1.z);
+  unpair(q[3], e2.x, e2.y);
+  e2.z = __ldg(reinterpret_cast<const float*>(t) + 8);
+}
+
+// The reference's triangle test (tri_hit, trace.wgsl:780-804): false when the
+// ray misses; u, v and t otherwise.
+template <bool ANY>
+__device__ __forceinline__ bool tri_test(v3 o, v3 d, v3 a, v3 e1, v3 e2, float inv_det, uint32_t word, float& u,
+                                         float& v, float& t) {
+  v3 pv = cross3(d, e2);
+  float det = dot3(e1, pv);
+  float seen = det * inv_det;
+  if (fabsf(seen) < 1e-9f) return false;
+  if (!ANY && (word & ONE_SIDED) != 0u && seen < 0.0f) return false;
+  float inv = 1.0f / det;
+  v3 sv = sub3(o, a);
+  u = dot3(sv, pv) * inv;
+  if (u < 0.0f || u > 1.0f) return false;
+  v3 qv = cross3(sv, e1);
+  v = dot3(d, qv) * inv;
+  if (v < 0.0f || u + v > 1.0f) return false;
+  t = dot3(e2, qv) * inv;
+  return true;
+}
+
+// One query's traversal state on the two-box nodes; the stack is the caller's.
+template <bool ANY, bool COUNT, int BOX = BOX_EITHER>
 struct Walker {
   TRay ray;     // ray in the current space (the world ray itself is the caller's: see inner_phase)
-  PRay pr;      // BOX_PAIRED: `ray` paired for the box test
   float limit;
   uint32_t base, record, word;
   float inv_det;
   uint32_t ref;
   float near_cur;
   int top;
-  uint32_t held;  // SPEC: the leaf set aside, REF_NONE when none
   bool done;
-  bool retry;  // BOX_BOUNDED, BOX_PAIRED: the ray is not bounded (or, paired, has a degenerate axis); walk
-               // it again with BOX_IEEE
   TraceHit hit;
   TraceCounts counts;
 
@@ -407,21 +373,7 @@ struct Walker {
     ref = s.root;
     near_cur = -INFINITY;
     top = 0;
-    held = REF_NONE;
     done = (s.root == REF_NONE);
-    retry = false;
-    if (BOX == BOX_BOUNDED && !done && !ray.bounded) {
-      retry = true;
-      done = true;
-    }
-    if (BOX == BOX_PAIRED && !done) {
-      if (!packable(ray)) {
-        retry = true;
-        done = true;
-      } else {
-        pr = make_pray(ray);
-      }
-    }
     hit.t = lim;
     hit.slot = hit.record = hit.hit = 0u;
     hit.u = hit.v = 0.0f;
@@ -446,16 +398,10 @@ struct Walker {
   template <class Stack, class World>
   __device__ __forceinline__ void inner_phase(const SceneView& s, Stack& st, const World& world) {
     while (!done) {
-      if constexpr (SPEC) {
-        // a lane holding a leaf walks on only while another lane of the warp still looks for one
-        if (held != REF_NONE && !__any_sync(__activemask(), held == REF_NONE)) return;
-      }
       if (ref == STACK_SENTINEL) {
-        if (SPEC && held != REF_NONE) return;  // the held leaf is tested in its own space
         v3 o, d;
         world(o, d);
         ray = make_tray(o, d, s.small);
-        if (BOX == BOX_PAIRED) pr = make_pray(ray);
         base = record = word = 0u;
         inv_det = 1.0f;
         pop(st);
@@ -469,38 +415,17 @@ struct Walker {
         const float4* p = reinterpret_cast<const float4*>(s.wide + ref);
         uint4 q3 = __ldg(reinterpret_cast<const uint4*>(p + 3));
         float n0 = 0.0f, n1 = 0.0f;
-        bool ok0, ok1;
         bool has1 = q3.y != REF_NONE;
-        if constexpr (BOX == BOX_PAIRED) {
-          // the node's twelve coordinates as six pairs: (lx, ly), (lz, hx), (hy, hz) of each child
-          const ulonglong2* pp = reinterpret_cast<const ulonglong2*>(p);
-          ulonglong2 a = __ldg(pp + 0), b = __ldg(pp + 1), c = __ldg(pp + 2);
-          ok0 = box_geometry_paired(a.x, a.y, b.x, pr, n0) && n0 <= hit.t;
-          ok1 = has1 && box_geometry_paired(b.y, c.x, c.y, pr, n1) && n1 <= hit.t;
-        } else {
-          float4 q0 = __ldg(p + 0), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
-          ok0 = box_test<BOX>(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, ray, n0) && n0 <= hit.t;
-          ok1 = has1 && box_test<BOX>(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, ray, n1) && n1 <= hit.t;
-        }
+        float4 q0 = __ldg(p + 0), q1 = __ldg(p + 1), q2 = __ldg(p + 2);
+        bool ok0 = box_test<BOX>(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, ray, n0) && n0 <= hit.t;
+        bool ok1 = has1 && box_test<BOX>(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, ray, n1) && n1 <= hit.t;
         if (COUNT) counts.boxes += 1u;  // the left child, popped next by the reference
-        uint32_t r0 = q3.x, r1 = q3.y;
-        if constexpr (ANY && !COUNT && TRACE_ANY_NEAR) {
-          // any hit: whether the ray is blocked does not depend on the order,
-          // so the nearer child goes first
-          if (ok0 && ok1 && n1 < n0) {
-            r0 = q3.y;
-            r1 = q3.x;
-            float t = n0;
-            n0 = n1;
-            n1 = t;
-          }
-        }
-        if ((ok1 || (COUNT && has1)) && top < (int)REF_STACK) {
-          st.put(top, r1, ok1 ? n1 : INFINITY);
+        if ((ok1 || (COUNT && has1)) && top < Stack::CAPACITY) {
+          st.put(top, q3.y, ok1 ? n1 : INFINITY);
           ++top;
         }
         if (ok0) {
-          ref = r0;
+          ref = q3.x;
           near_cur = n0;
         } else {
           pop(st);
@@ -508,8 +433,7 @@ struct Walker {
         continue;
       }
       if ((ref & REF_INST) == REF_INST) {
-        if (SPEC && held != REF_NONE) return;  // the held leaf is tested in its own space
-        if (top >= (int)REF_STACK) {  // refused at creation; never taken
+        if (top >= Stack::CAPACITY) {  // refused at creation; never taken
           pop(st);
           continue;
         }
@@ -527,115 +451,30 @@ struct Walker {
           v3 o, d;
           world(o, d);
           ray = make_tray(to_object(r0, r1, r2, o, 1.0f), to_object(r0, r1, r2, d, 0.0f), s.small);
-          if (BOX == BOX_BOUNDED && !ray.bounded) {
-            retry = true;
-            done = true;
-            return;
-          }
-          if (BOX == BOX_PAIRED) {
-            if (!packable(ray)) {
-              retry = true;
-              done = true;
-              return;
-            }
-            pr = make_pray(ray);
-          }
         }
         ref = m.x;
         near_cur = -INFINITY;
         continue;
       }
-      // a leaf that passed its near check
-      if constexpr (SPEC) {
-        if (held == REF_NONE) {
-          held = ref;
-          prefetch_leaf(s, ref);
-          pop(st);
-          continue;
-        }
-      }
-      return;
+      return;  // a leaf that passed its near check
     }
   }
 
-  // A leaf set aside is tested later: its triangles (contiguous TravTri
-  // records, 48 bytes each) may be fetched meanwhile.
-  __device__ __forceinline__ void prefetch_leaf(const SceneView& s, uint32_t leaf) const {
-#if TRACE_LEAF_PREFETCH
-    const uint32_t n = ((leaf >> LEAF_FIRST_BITS) & 15u) + 1u;
-    const char* p = reinterpret_cast<const char*>(s.tris + base + (leaf & LEAF_FIRST_MASK));
-#if TRACE_LEAF_PREFETCH == 1
-    for (uint32_t b = 0; b < n * 48u; b += 128u) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + b));
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + n * 48u - 1u));
-#else
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(n * 48u) : "memory");
-#endif
-#else
-    (void)s;
-    (void)leaf;
-#endif
-  }
-
-  // SPEC: is there a leaf to test (the held one, or the current entry)?
-  __device__ __forceinline__ bool leaf_ready() const { return SPEC ? (held != REF_NONE || !done) : !done; }
-
-  // Test the triangles of the held leaf, then move to the next entry.
+  // Test the triangles of the current leaf, then move to the next entry.
   template <class Stack>
   __device__ __forceinline__ void leaf_phase(const SceneView& s, Stack& st) {
-    // SPEC: the held leaf first; the current entry stays, to be checked again
-    const bool from_held = SPEC && held != REF_NONE;
-    const uint32_t leaf = from_held ? held : ref;
-    if (SPEC) held = REF_NONE;
-    uint32_t first = leaf & LEAF_FIRST_MASK;
-    uint32_t n = ((leaf >> LEAF_FIRST_BITS) & 15u) + 1u;
+    uint32_t first = ref & LEAF_FIRST_MASK;
+    uint32_t n = ((ref >> LEAF_FIRST_BITS) & 15u) + 1u;
     bool skip = ANY ? ((word & CASTS_NO_SHADOW) != 0u) : ((word & SHADOW_ONLY) != 0u);
     if (COUNT && skip) counts.tris += n;
     if (!skip) {
       for (uint32_t j = 0; j < n; ++j) {
         if (COUNT) counts.tris += 1u;  // the reference stops counting at an any-hit blocker
         uint32_t i = base + first + j;
-        const float4* tp = reinterpret_cast<const float4*>(s.tris + i);
-        float4 ta = __ldg(tp + 0), te1 = __ldg(tp + 1), te2 = __ldg(tp + 2);
-        v3 a = mk3(ta.x, ta.y, ta.z), e1 = mk3(te1.x, te1.y, te1.z), e2 = mk3(te2.x, te2.y, te2.z);
+        v3 a, e1, e2;
+        load_tri(s.tris + i, a, e1, e2);
         float u, v, t;
-        if constexpr (BOX == BOX_PAIRED) {
-          // The same test on the negated direction n = -d the paired ray
-          // holds: pv, det and inv change sign exactly (round-to-nearest is
-          // symmetric), so u and v are the same bits and t = -(e2.qv * inv).
-          v3 rn, ro;
-          float spare;
-          unpair(pr.nd[0], rn.x, rn.y);
-          unpair(pr.nd[1], rn.z, spare);
-          unpair(pr.o[0], ro.x, ro.y);
-          unpair(pr.o[1], ro.z, spare);
-          v3 pv = cross3(rn, e2);
-          float det = dot3(e1, pv);
-          float seen = det * inv_det;
-          if (fabsf(seen) < 1e-9f) continue;
-          if (!ANY && (word & ONE_SIDED) != 0u && seen > 0.0f) continue;
-          float inv = 1.0f / det;
-          v3 sv = sub3(ro, a);
-          u = dot3(sv, pv) * inv;
-          if (u < 0.0f || u > 1.0f) continue;
-          v3 qv = cross3(sv, e1);
-          v = dot3(rn, qv) * inv;
-          if (v < 0.0f || u + v > 1.0f) continue;
-          t = -(dot3(e2, qv) * inv);
-        } else {
-          v3 pv = cross3(ray.d, e2);
-          float det = dot3(e1, pv);
-          float seen = det * inv_det;
-          if (fabsf(seen) < 1e-9f) continue;
-          if (!ANY && (word & ONE_SIDED) != 0u && seen < 0.0f) continue;
-          float inv = 1.0f / det;
-          v3 sv = sub3(ray.o, a);
-          u = dot3(sv, pv) * inv;
-          if (u < 0.0f || u > 1.0f) continue;
-          v3 qv = cross3(sv, e1);
-          v = dot3(ray.d, qv) * inv;
-          if (v < 0.0f || u + v > 1.0f) continue;
-          t = dot3(e2, qv) * inv;
-        }
+        if (!tri_test<ANY>(ray.o, ray.d, a, e1, e2, inv_det, word, u, v, t)) continue;
         if (ANY) {
           if (t <= 0.0001f || t >= limit) continue;
           hit.hit = 1u;
@@ -654,24 +493,331 @@ struct Walker {
         }
       }
     }
-    if (!from_held) pop(st);
+    pop(st);
   }
 
   // Run to completion (one query, no work sharing).
   template <class Stack, class World>
   __device__ __forceinline__ void run(const SceneView& s, Stack& st, const World& world) {
-    while (leaf_ready()) {
+    while (!done) {
       inner_phase(s, st, world);
-      if (!leaf_ready()) break;
-      leaf_phase(s, st);
+      if (!done) leaf_phase(s, st);
     }
+  }
+};
+
+// The walk of the batch and queue kernels, on the four-box nodes.
+//
+// What it may skip.  The reference tests a leaf's triangles when the leaf's box
+// and every ancestor's passed, each against the hit distance at its turn.  The
+// fp32 quotients are monotone in the plane, so in one space a box that passes
+// implies that the boxes holding it pass, with entries no larger, and hit
+// distances only shrink: the leaf's own exact test at its turn decides alone
+// (and, for an instance, the instance leaf's in world space).  Every box on
+// the way down may therefore be skipped or tested loosely, as long as nothing
+// that holds a passing leaf is dropped.
+//
+// The loose test.  A plane's quotient is x * r with x = lo - o rounded as the
+// reference rounds it and r within an ulp of 1/d: within 2^-21 of the
+// reference's quotient x / d in relative terms for a bounded ray (no
+// underflow), and the planes a ray enters and leaves through follow from the
+// signs of d (lo <= hi).  Entry <= exit and entry <= hit.t are compared with
+// the right side scaled by 1 + 2^-18, so a box that passes exactly passes here.
+//
+// The exact test (box_exact) runs where it decides: before the first triangle
+// of a leaf is accepted, against the hit distance from before that leaf, and
+// when an instance is entered.
+//
+// What bounds it.  The two-box walk spent 24 instructions on each box and, at
+// 10 to 13 of 32 lanes, issue slots (70 % busy).  Four boxes a visit, tested
+// loosely, and votes that name every lane leave half the warp instructions at
+// 18 to 20 lanes, and the L1's handling of divergent sectors (84 % busy for
+// shadow rays) bounds it: hence planes stored so that one 32-byte load brings
+// a whole sector of an axis, four loads a node (with six 16-byte loads of the
+// planes that the ray's signs pick: 1897 and 1048 us instead of 1797 and 925).
+// Start to now, one B200: room closest 2^21 rays 2646 -> 1797 us, room any
+// 1.5 M rays 1100 -> 925 us, instanced closest and any 0.5 M rays 476 -> 355
+// and 518 -> 403 us.  32 resident warps (64 registers) beat 24, 28, 36 and 40.
+//
+// Order.  Children are visited in the reference's left-first order and a
+// popped entry is checked again against the current distance, so the leaves
+// tested, their order and the distance at each are the reference's.  A lane
+// that reaches a leaf while other lanes of its warp still walk inner nodes
+// sets the leaf aside (`held`) and walks on, so that the warp's leaf tests run
+// with more lanes at once (Aila and Laine, "Understanding the efficiency of
+// ray traversal on GPUs", 2009): the held leaf is the next one in the
+// reference's order and is tested before any other, and what the lane walked
+// past it was decided against a distance no smaller than the reference's.  A
+// held leaf is tested before the walk enters or leaves an instance, so it is
+// tested in its own space.
+constexpr float LOOSE = 1.0f + 0x1p-18f;
+// Lanes with a leaf set aside that send the warp to its leaf tests.  Measured
+// (us; room closest 2^21 rays, room any 1.5 M, instanced closest and any 0.5 M):
+// only when nobody looks any more 1922, 1072, 377, 445; 12 lanes 1970, 1060,
+// 341, 401; 16 lanes 1897, 1048, 343, 410; 20 lanes 1867, 1041, 358, 420; as
+// many as still look 1984, 1043, 334, 392 (16-byte node loads).
+constexpr int HOLDERS = 16;
+
+template <bool ANY>
+struct QuadWalker {
+  // the ray of the current space: origins and approximate reciprocals in both
+  // lanes of a pair (a node's planes come two children to a pair), the
+  // direction, and per axis the byte offset in a node of the planes it enters
+  // through
+  f32x2 ox, oy, oz, rx, ry, rz;
+  v3 d;
+  uint32_t inst;  // the instance the walk is in, REF_NONE in world space
+  uint32_t ref;   // the entry at hand, REF_NONE when there is none
+  float near_cur;
+  int top;
+  uint32_t held;  // the leaf set aside, REF_NONE when none
+  TraceHit hit;   // any hit: t stays the limit; record: the instance until `record()` gives its record
+
+  static constexpr uint32_t RETRY = 2u;  // hit.hit of a ray to be walked again with BOX_IEEE: not bounded, or
+                                         // with a degenerate axis, in world or instance space
+
+  // A lane without a ray.
+  __device__ __forceinline__ void idle() { ref = held = REF_NONE; }
+
+  // False when the ray cannot be taken (the walk is then over).
+  __device__ __forceinline__ bool aim(const SceneView& s, v3 o, v3 dir) {
+    if (!(s.small != 0u && bounded_axis(o.x, dir.x) && bounded_axis(o.y, dir.y) && bounded_axis(o.z, dir.z) &&
+          fabsf(dir.x) >= 1e-12f && fabsf(dir.y) >= 1e-12f && fabsf(dir.z) >= 1e-12f)) {
+      hit.hit = RETRY;
+      ref = REF_NONE;
+      return false;
+    }
+    ox = pair(o.x, o.x);
+    oy = pair(o.y, o.y);
+    oz = pair(o.z, o.z);
+    const float r0 = rcp_approx(dir.x), r1 = rcp_approx(dir.y), r2 = rcp_approx(dir.z);
+    rx = pair(r0, r0);
+    ry = pair(r1, r1);
+    rz = pair(r2, r2);
+    d = dir;
+    return true;
+  }
+
+  __device__ __forceinline__ void start(const SceneView& s, v3 wo, v3 wd, float lim) {
+    inst = REF_NONE;
+    ref = s.root;
+    near_cur = -INFINITY;
+    top = 0;
+    held = REF_NONE;
+    hit.t = lim;
+    hit.slot = hit.hit = 0u;
+    hit.record = REF_NONE;
+    hit.u = hit.v = 0.0f;
+    if (ref != REF_NONE) aim(s, wo, wd);
+  }
+
+  // The surface record of the hit (0: the world's, or no hit).
+  __device__ __forceinline__ uint32_t record(const SceneView& s) const {
+    return hit.record == REF_NONE ? 0u : __ldg(&s.insts[hit.record].record);
+  }
+
+  // The next entry that the current hit distance leaves.
+  template <class Stack>
+  __device__ __forceinline__ void pop(const Stack& st) {
+    do {
+      if (top == 0) {
+        ref = REF_NONE;
+        return;
+      }
+      --top;
+      st.get(top, ref, near_cur);
+    } while (!(near_cur <= hit.t * LOOSE));
+  }
+
+  __device__ __forceinline__ v3 origin() const {
+    float x, y, z, spare;
+    unpair(ox, x, spare);
+    unpair(oy, y, spare);
+    unpair(oz, z, spare);
+    return mk3(x, y, z);
+  }
+
+  // The reference's test of one box (box_geometry_bounded for a ray without a
+  // degenerate axis) against the hit distance `reach`.
+  __device__ __forceinline__ bool box_exact(float lx, float ly, float lz, float hx, float hy, float hz,
+                                            float reach) const {
+    const v3 o = origin();
+    float r = 1.0f / d.x;
+    float a = quotient(lx - o.x, d.x, r), b = quotient(hx - o.x, d.x, r);
+    float n = fmaxf(0.0f, fminf(a, b)), f = fmaxf(a, b);
+    r = 1.0f / d.y;
+    a = quotient(ly - o.y, d.y, r), b = quotient(hy - o.y, d.y, r);
+    n = fmaxf(n, fminf(a, b)), f = fminf(f, fmaxf(a, b));
+    r = 1.0f / d.z;
+    a = quotient(lz - o.z, d.z, r), b = quotient(hz - o.z, d.z, r);
+    n = fmaxf(n, fminf(a, b)), f = fminf(f, fmaxf(a, b));
+    return !(n > f) && n <= reach;
+  }
+
+  // Opens the inner node at hand: tests its four children loosely; the first
+  // that passes is next, the others are pushed last first.
+  template <class Stack>
+  __device__ __forceinline__ void open(const SceneView& s, Stack& st) {
+    const char* p = reinterpret_cast<const char*>(s.quad + ref);
+    const uint4 c = __ldg(reinterpret_cast<const uint4*>(p + 96));
+    f32x2 x[4], y[4], z[4];  // lo of children 0-1 and 2-3, hi of 0-1 and 2-3
+    load32(p, x);
+    load32(p + 32, y);
+    load32(p + 64, z);
+    uint32_t next = REF_NONE;
+    float next_near = 0.0f;
+#pragma unroll
+    for (int h = 1; h >= 0; --h) {
+      float xl[2], yl[2], zl[2], xh[2], yh[2], zh[2];
+      unpair(mul2(sub2(x[h], ox), rx), xl[0], xl[1]);
+      unpair(mul2(sub2(y[h], oy), ry), yl[0], yl[1]);
+      unpair(mul2(sub2(z[h], oz), rz), zl[0], zl[1]);
+      unpair(mul2(sub2(x[2 + h], ox), rx), xh[0], xh[1]);
+      unpair(mul2(sub2(y[2 + h], oy), ry), yh[0], yh[1]);
+      unpair(mul2(sub2(z[2 + h], oz), rz), zh[0], zh[1]);
+#pragma unroll
+      for (int k = 1; k >= 0; --k) {
+        const float entry = fmaxf(max3f(fminf(xl[k], xh[k]), fminf(yl[k], yh[k]), fminf(zl[k], zh[k])), 0.0f);
+        const float exit = fminf(min3f(fmaxf(xl[k], xh[k]), fmaxf(yl[k], yh[k]), fmaxf(zl[k], zh[k])), hit.t);
+        if (entry <= exit * LOOSE) {
+          if (next != REF_NONE) st.put(top++, next, next_near);
+          next = h ? (k ? c.w : c.z) : (k ? c.y : c.x);
+          next_near = entry;
+        }
+      }
+    }
+    if (next != REF_NONE) {
+      ref = next;
+      near_cur = next_near;
+    } else {
+      pop(st);
+    }
+  }
+
+  // Whether the entry at hand enters or leaves an instance.
+  __device__ __forceinline__ bool at_instance() const {
+    return ref != REF_NONE && (ref & REF_INST) == REF_INST;
+  }
+  static_assert((STACK_SENTINEL & REF_INST) == REF_INST, "the sentinel is told from leaves by the instance bits");
+
+  // Sets the leaf at hand aside.
+  template <class Stack>
+  __device__ __forceinline__ void take_leaf(const Stack& st) {
+    if (held == REF_NONE && (ref & REF_INST) == REF_LEAF) {
+      held = ref;
+      pop(st);
+    }
+  }
+
+  // Enters or leaves the instance at hand.  Only without a held leaf, which is
+  // tested in its own space.
+  template <class Stack, class World>
+  __device__ __forceinline__ void cross_instance(const SceneView& s, Stack& st, const World& world) {
+    if (ref == STACK_SENTINEL) {
+      v3 o, dir;
+      world(o, dir);
+      aim(s, o, dir);
+      inst = REF_NONE;
+      pop(st);
+      return;
+    }
+    const uint32_t index = ref & 0x3fffffffu;
+    const float4* p = reinterpret_cast<const float4*>(s.insts + index);
+    const uint32_t root = __ldg(reinterpret_cast<const uint32_t*>(p + 3));
+    const float4 m2 = __ldg(p + 4), m3 = __ldg(p + 5);
+    if (!box_exact(m2.z, m2.w, m3.x, m3.y, m3.z, m3.w, hit.t)) {
+      pop(st);
+      return;
+    }
+    st.put(top++, STACK_SENTINEL, -INFINITY);
+    inst = index;
+    ref = root;
+    near_cur = -INFINITY;
+    if (__float_as_uint(m2.y) != 0u) {
+      const float4 r0 = __ldg(p + 0), r1 = __ldg(p + 1), r2 = __ldg(p + 2);
+      v3 o, dir;
+      world(o, dir);
+      aim(s, to_object(r0, r1, r2, o, 1.0f), to_object(r0, r1, r2, dir, 0.0f));
+    }
+  }
+
+  // Walks every lane's inner nodes until enough lanes hold a leaf; called by
+  // all 32 lanes.  world(o, d): as Walker::inner_phase.  The votes name every
+  // lane, so the warp takes each step together: with votes among whichever
+  // lanes had come together, a warp fell apart (5.4 lanes an instruction
+  // against 8.6 on a small frame's rays).
+  template <class Stack, class World>
+  __device__ __forceinline__ void inner_phase(const SceneView& s, Stack& st, const World& world) {
+    constexpr unsigned FULL = 0xffffffffu;
+    for (;;) {
+      take_leaf(st);
+      if (__any_sync(FULL, at_instance() && held == REF_NONE)) {
+        if (at_instance() && held == REF_NONE) cross_instance(s, st, world);
+        continue;
+      }
+      const bool inner = (ref & REF_LEAF) == 0u;
+      // Lanes that hold a leaf walk on while others still look for one, until
+      // half the warp holds one or nobody looks any more.
+      const unsigned look = __ballot_sync(FULL, inner && held == REF_NONE);
+      if (look == 0u) break;
+      if (__popc(__ballot_sync(FULL, held != REF_NONE)) >= HOLDERS) break;
+      if (inner) open(s, st);
+    }
+  }
+
+  // Is there a leaf to test?  Without one, inner_phase has ended the walk.
+  __device__ __forceinline__ bool leaf_ready() const { return held != REF_NONE; }
+  __device__ __forceinline__ bool finished() const { return ref == REF_NONE && held == REF_NONE; }
+
+  // Test the triangles of the held leaf; the entry at hand stays, checked
+  // again against the new distance.
+  template <class Stack>
+  __device__ __forceinline__ void leaf_phase(const SceneView& s, Stack& st) {
+    uint32_t i = held & LEAF_FIRST_MASK, word = 0u;
+    const uint32_t n = ((held >> LEAF_FIRST_BITS) & 15u) + 1u;
+    float inv_det = 1.0f;
+    held = REF_NONE;
+    if (inst != REF_NONE) {
+      const InstRec* r = s.insts + inst;
+      i += __ldg(&r->base);
+      word = __ldg(&r->word);
+      inv_det = __ldg(&r->inv_det);
+      if (ANY ? ((word & CASTS_NO_SHADOW) != 0u) : ((word & SHADOW_ONLY) != 0u)) return;
+    }
+    const float reach = hit.t;
+    const v3 o = origin();
+    bool checked = false;
+    for (const uint32_t end = i + n; i < end; ++i) {
+      const TravTri* tri = s.tris + i;
+      v3 a, e1, e2;
+      load_tri(tri, a, e1, e2);
+      float u, v, t;
+      if (!tri_test<ANY>(o, d, a, e1, e2, inv_det, word, u, v, t)) continue;
+      if (ANY ? (t <= 0.0001f || t >= hit.t) : !(t > 0.0001f && t < hit.t)) continue;
+      if (!checked) {
+        const float* b = tri->lo;
+        if (!box_exact(__ldg(b), __ldg(b + 1), __ldg(b + 2), __ldg(b + 3), __ldg(b + 4), __ldg(b + 5), reach)) return;
+        checked = true;
+      }
+      hit.hit = 1u;
+      if (ANY) {
+        ref = REF_NONE;
+        return;
+      }
+      hit.t = t;
+      hit.slot = i;
+      hit.record = inst;
+      hit.u = u;
+      hit.v = v;
+    }
+    if (ref != REF_NONE && !(near_cur <= hit.t * LOOSE)) pop(st);
   }
 };
 
 // Single-query helpers used by shading code.
 template <bool ANY>
 __device__ __forceinline__ TraceHit traverse(const SceneView& s, v3 o, v3 d, float limit) {
-  LaneStack<0> st;
+  RefStack st;
   Walker<ANY, false, BOX_EITHER> w;
   w.start(s, o, d, limit);
   w.run(s, st, [&](v3& wo, v3& wd) {

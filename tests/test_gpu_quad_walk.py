@@ -1,0 +1,105 @@
+"""The four-box walk at the sizes and rays where it can go wrong: trees of one
+to a few nodes, trees that are one long chain, flat boxes, every class of ray
+it hands over (degenerate axes, long directions, far origins) and limits that
+are zero, negative, infinite or NaN, against the oracle bit for bit."""
+import numpy as np
+import pytest
+
+import oracle
+from pfx_b200 import synth
+from pfx_b200.trace import SceneDesc, Settings, Trace, make_rays
+
+F32 = np.float32
+
+
+def rays_for(rng, lo, hi, n):
+    o = rng.uniform(lo, hi, (n, 3)).astype(F32)
+    d = rng.normal(size=(n, 3)).astype(F32)
+    k = np.arange(n)
+    d[k % 7 == 1, 0] = 0.0                      # degenerate axes
+    d[k % 7 == 2, 1:] = 0.0
+    d[k % 14 == 3] *= F32(3e6)                  # beyond the bounded directions
+    d[k % 14 == 10, 2] = F32(-0.0)
+    o[k % 28 == 4, 0] = F32(1e25)               # beyond the bounded origins
+    o[k % 11 == 5] = np.round(o[k % 11 == 5])   # origins on box planes
+    return o, d
+
+
+def compare(trace, ref, batch):
+    got = trace.trace_rays(batch)
+    want = oracle.trace(ref, batch)
+    assert np.array_equal(got["hit"], want["hit"])
+    h = want["hit"] == 1
+    assert np.array_equal(got["slot"][h], want["slot"][h])
+    assert np.array_equal(got["record"][h], want["record"][h])
+    assert np.array_equal(got["t"][h].view(np.uint32), want["t"][h].view(np.uint32))
+    assert np.array_equal(trace.occluded(batch), oracle.trace(ref, batch, any_hit=True)["hit"] == 1)
+    return h.sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 5, 9, 17, 40, 300])
+@pytest.mark.parametrize("shape", ["cloud", "flat", "chain"])
+def test_small_trees(gpu, count, shape):
+    rng = np.random.default_rng(count)
+    v = rng.uniform(-4, 4, (count, 1, 3)) + rng.uniform(-1.5, 1.5, (count, 3, 3))
+    if shape == "flat":       # boxes of no thickness, corners on whole numbers, some shared
+        v = np.round(v)
+        v[:, :, count % 3] = np.round(v[:, :1, count % 3])
+    if shape == "chain":      # triangles at ever larger distances: a tree that is one long chain
+        v = (v * 0.1 + 1.0) * (1.3 ** np.arange(count) if count < 150 else 1.05 ** np.arange(count))[:, None, None]
+    scene = SceneDesc(synth.triangles(v.astype(F32)), synth.material(), synth.look_at((0, 0, 10), (0, 0, 0), 45, 1.0))
+    trace = Trace(scene, Settings(), 8, 8)
+    ref = oracle.scene_buffers(scene, Settings())
+    top = float(np.abs(v).max())
+    o, d = rays_for(rng, -top, top, 3000)
+    aim = v[rng.integers(0, count, 3000)].mean(1).astype(F32)   # half of them towards a triangle
+    d[::2] = (aim - o)[::2]
+    hits = compare(trace, ref, make_rays(o, d, 1e20))
+    assert hits > 0 or count < 9   # rounded to whole numbers, a few triangles may all be degenerate
+    for limit in (0.0, -1.0, 1e-3, 0.5, np.inf):
+        compare(trace, ref, make_rays(o, d, F32(limit)))
+    nan = make_rays(o, d, F32(np.nan))
+    assert not trace.occluded(nan).any() and not trace.trace_rays(nan)["hit"].any()
+
+
+@pytest.mark.gpu
+def test_instances_with_every_ray_class(gpu):
+    w = synth.instanced_1080(target=3000)
+    trace = Trace(w.scene, w.settings, 8, 8)
+    ref = oracle.scene_buffers(w.scene, w.settings)
+    rng = np.random.default_rng(2)
+    o, d = rays_for(rng, (-60, 0, -60), (60, 40, 60), 20000)
+    assert compare(trace, ref, make_rays(o, d, 1e20)) > 1000
+    compare(trace, ref, make_rays(o, d, rng.uniform(0.0, 60.0, len(o)).astype(F32)))
+
+
+def test_the_loose_comparison_holds_every_box_that_passes_exactly():
+    """Entry and exit by x * r with r an ulp off 1/d, the comparison scaled by
+    1 + 2^-18, against the quotients (fp32 arithmetic, worst cases of r)."""
+    rng = np.random.default_rng(9)
+    n = 400_000
+    o = rng.normal(size=(n, 3)).astype(F32) * F32(10.0) ** rng.integers(-3, 4, (n, 1)).astype(F32)
+    lo = (o + rng.normal(size=(n, 3)).astype(F32) * F32(10.0) ** rng.integers(-4, 3, (n, 1)).astype(F32)).astype(F32)
+    size = np.abs(rng.normal(size=(n, 3))).astype(F32) * F32(10.0) ** rng.integers(-6, 2, (n, 3)).astype(F32)
+    size[rng.random((n, 3)) < 0.2] = 0.0
+    hi = (lo + size).astype(F32)
+    aim = (lo + size * rng.choice([0.0, 0.5, 1.0], (n, 3)).astype(F32)).astype(F32)  # at the corners and edges
+    d = (aim - o).astype(F32)
+    d = (d.view(np.int32) + rng.integers(-3, 4, (n, 3)).astype(np.int32)).view(F32)  # and a few ulps beside them
+    ok = ((np.abs(d) >= 1e-12) & (np.abs(d) < 1e6)).all(1)
+    o, lo, hi, d = o[ok], lo[ok], hi[ok], d[ok]
+    a, b = (lo - o) / d, (hi - o) / d
+    near = np.maximum(np.minimum(a, b).max(1), F32(0))
+    far = np.maximum(a, b).min(1)
+    exact = ~(near > far)
+    assert 0.2 < exact.mean() < 1.0
+    for ulps in (-1, 0, 1):
+        r = F32(1.0) / d
+        r = (r.view(np.int32) + np.int32(ulps)).view(F32)
+        a, b = (lo - o) * r, (hi - o) * r
+        n_l = np.maximum(np.minimum(a, b).max(1), F32(0))
+        f_l = np.maximum(a, b).min(1)
+        scale = F32(1.0) + F32(2.0) ** F32(-18)
+        for limit in (np.full_like(near, np.inf), near):   # the tightest limit that the box passes
+            assert (n_l <= np.minimum(f_l, limit) * scale)[exact].all()
