@@ -2,7 +2,9 @@
 // sequence of kernels over path queues instead of the reference's megakernel
 // main() (trace.wgsl:2503-2579).
 //
-// One wave traces one sample for every active pixel.  Per bounce:
+// One wave traces 2^shift samples of every active pixel (as many as a call
+// asks for and the wave holds: path i is sample i mod 2^shift of active pixel
+// i >> shift).  Per bounce:
 //   extend   closest hit of every queued path (persistent traversal kernel)
 //   shade    the body of radiance()'s bounce loop (trace.wgsl:2169-2500):
 //            emission, light selection and BSDF sampling; writes up to `cap`
@@ -14,8 +16,9 @@
 // the start of the path's next shade (or in finish), in light-slot order, so
 // the result is summed in exactly the reference's order; with the draws of
 // the reference's random sequence kept in order, a pixel's value equals the
-// reference's bit for bit.  Waves run in sample order, so the accumulation of
-// samples into the 48 B/pixel Accum also keeps the reference's order.
+// reference's bit for bit.  Waves run in sample order and a wave's samples of a
+// pixel are added in theirs, so the accumulation of samples into the 48 B/pixel
+// Accum also keeps the reference's order.
 //
 // Zero-valued light-slot contributions (a black sky, a light behind the
 // surface) add nothing and trace no shadow ray; their random draws are still
@@ -126,7 +129,9 @@ struct Pass {
   SceneView s;
   Wave w;
   CachePass c;
-  uint32_t sample;     // sample index inside the pass
+  uint32_t sample;     // sample index inside the pass of the wave's first sample
+  uint32_t shift;      // log2 of the samples of a pixel in the wave
+  uint32_t capacity;   // paths the wave's buffers hold
   uint32_t bounce;
   uint32_t cap;        // shadow slots per path
   uint32_t deferred;   // 1: light-slot shadow rays go through the shadow queue
@@ -150,6 +155,16 @@ __device__ __forceinline__ uint32_t pass_seed(const Pass& P) { return __ldg(P.va
 __device__ __forceinline__ v3 pass_camera(const Pass& P, int k) {
   float4 c = __ldg(reinterpret_cast<const float4*>(P.vars) + 1 + k);
   return mk3(c.x, c.y, c.z);
+}
+
+// The wave's paths: its samples of every active pixel.  (The host chooses the
+// shift so that they fit; the bound keeps every index inside the buffers.)
+__device__ __forceinline__ uint32_t wave_paths(const Pass& P) {
+  return min(P.w.counters[3], P.capacity >> P.shift) << P.shift;
+}
+// Sample index inside the pass of path i.
+__device__ __forceinline__ uint32_t path_sample(const Pass& P, uint32_t i) {
+  return P.sample + (i & ((1u << P.shift) - 1u));
 }
 
 // The fallback grid: may a path end into the cache at p?
@@ -213,14 +228,14 @@ __global__ void k_collect(const __grid_constant__ Pass P,const Accum* __restrict
 // ------------------------------------------------------------------ generate
 // main() up to the call of radiance(): seeding, pixel filter, camera ray.
 __global__ void k_gen(const __grid_constant__ Pass P) {
-  const uint32_t n = P.w.counters[3];
+  const uint32_t n = wave_paths(P);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    uint32_t pixel = P.w.active[i];
+    uint32_t pixel = P.w.active[i >> P.shift];
     uint32_t gx = pixel % P.width, gy = pixel / P.width;
     uint32_t px = gx + P.f.window[2], py = gy + P.f.window[3];
     uint32_t stream = py * P.f.window[0] + px;
     const uint32_t seed = pass_seed(P);
-    uint32_t absolute = pass_accum(P) + P.sample;
+    uint32_t absolute = pass_accum(P) + path_sample(P, i);
     uint32_t state = pcg(stream * 1973u + pcg(seed * 9277u + absolute * 7919u + 26699u));
     Rng r{hash_iqnt2d(px, py) ^ seed, absolute, 0u};
     float4 pf = sobol4(P.v, P.sp, r, 0u);
@@ -277,7 +292,7 @@ __global__ void k_cache_begin(const __grid_constant__ Pass P) {
 
 __global__ void k_seed_counts(const __grid_constant__ Pass P) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    P.w.counters[0] = P.w.counters[3];
+    P.w.counters[0] = wave_paths(P);
     P.w.counters[1] = 0u;
     P.w.counters[2] = 0u;
   }
@@ -662,7 +677,7 @@ __global__ void __launch_bounds__(kThreads, SHADE_MIN_BLOCKS) k_shade(const __gr
       flags &= ~(15u << F_PEND);
       uint32_t pixel = __float_as_uint(rs.w);
       uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
-      Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + P.sample, 16u * (bounce + 1u)};
+      Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (bounce + 1u)};
       float4 h = P.w.hit[i];
       float reach = h.x;
       v3 origin_point = spawn_point(o, neg3(d), o, 0.0f);
@@ -1018,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
     v3 result = mk3(rs.x, rs.y, rs.z);
     uint32_t pixel = __float_as_uint(rs.w);
     uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
-    Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + P.sample, 16u * (bounce + 1u)};
+    Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (bounce + 1u)};
     // The surface's geometry is held across the slots; its material record is
     // read again where a slot evaluates the BSDF, so that it is not live across
     // the light-tree descent (fewer values to keep in local memory there).
@@ -1160,9 +1175,10 @@ constexpr int SLOT_SUN = 0, SLOT_SKY = 1, SLOT_EMITTER = 2, SLOT_LOOPED = 3, SLO
 #define PICK_INLINE false
 #endif
 
-__device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t pixel) {
+__device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i) {
+  const uint32_t pixel = __float_as_uint(reinterpret_cast<const float*>(P.w.res + i)[3]);
   uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
-  return Rng{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + P.sample, 16u * (P.bounce + 1u)};
+  return Rng{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (P.bounce + 1u)};
 }
 
 // The light tree's descent for every scattering path (slot k of tree_pick's
@@ -1178,8 +1194,7 @@ __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const _
     uint32_t state = __float_as_uint(reinterpret_cast<const float*>(P.w.thr + i)[3]);
     float start;
     if (sp.sobol) {
-      start = sobol4(V, sp, slot_rng(P, __float_as_uint(reinterpret_cast<const float*>(P.w.res + i)[3])),
-                     light_dim(k)).z;
+      start = sobol4(V, sp, slot_rng(P, i), light_dim(k)).z;
     } else {
       start = random01(state);
       reinterpret_cast<float*>(P.w.thr + i)[3] = __uint_as_float(state);
@@ -1214,8 +1229,7 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
     const v3 p = mk3(g0.x, g0.y, g0.z), nn = mk3(g1.x, g1.y, g1.z);
     const m3 transform = basis(nn);
     float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (sp.sobol) u = sobol4(V, sp, slot_rng(P, __float_as_uint(reinterpret_cast<const float*>(P.w.res + i)[3])),
-                             light_dim(k));
+    if (sp.sobol) u = sobol4(V, sp, slot_rng(P, i), light_dim(k));
     v3 local = mk3(0.0f, 0.0f, 1.0f), direction = mk3(0.0f, 0.0f, 1.0f), strength = splat3(0.0f);
     v3 origin = p;
     float limit = 1e19f, pdf = 0.0f;
@@ -1330,7 +1344,7 @@ __global__ void __launch_bounds__(kThreads) k_shade_bsdf(const __grid_constant__
       uint32_t state = __float_as_uint(th.w);
       uint32_t pixel = __float_as_uint(P.w.res[i].w);
       uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
-      Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + P.sample, 16u * (bounce + 1u)};
+      Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (bounce + 1u)};
       const Surface S = load_surface_record(P.w.surf + (size_t)i * 9u);
       const Shaded& s = S.s;
       const v3 p = S.p;
@@ -1391,32 +1405,35 @@ __global__ void __launch_bounds__(kThreads) k_shade_bsdf(const __grid_constant__
 
 // ------------------------------------------------------------------ finish
 // Pending contributions of the last bounce, then Accum += (result, first
-// albedo, first normal) in sample order (trace.wgsl:2564-2567).
+// albedo, first normal) in sample order (trace.wgsl:2564-2567): one thread an
+// active pixel, over the wave's samples of it.
 __global__ void k_finish(const __grid_constant__ Pass P,Accum* __restrict__ accum) {
-  const uint32_t n = P.w.counters[3];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float4 rs = P.w.res[i];
-    uint32_t flags = __float_as_uint(P.w.ray_d[i].w);
-    v3 result = flush_pending(P, i, flags, mk3(rs.x, rs.y, rs.z));
-    if (flags & F_CACHED) {
-      // the cache's radiance at the vertex the path ended at, through its throughput
-      float4 pr = P.c.pred[i], th = P.w.thr[i];
-      v3 radiance = mk3(fmaxf(pr.x, 0.0f), fmaxf(pr.y, 0.0f), fmaxf(pr.z, 0.0f));
-      result = add3(result, capped(P, mul3(mk3(th.x, th.y, th.z), radiance), true));
-    }
-    if (P.c.enabled) {
-      uint32_t ts = P.c.tslot[i];
-      if (ts != ~0u)
-        emit_records(P.c.tvert, P.c.records, P.w.counters + 7, P.c.rcap, P.c.record_bounces + 1u, ts, result);
-    }
-    uint32_t pixel = __float_as_uint(rs.w);
+  const uint32_t n = wave_paths(P) >> P.shift;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const uint32_t pixel = P.w.active[k];
     Accum a = accum[pixel];
-    float4 al = P.w.alb[i], nr = P.w.nrm[i];
-    a.color.x = a.color.x + result.x;
-    a.color.y = a.color.y + result.y;
-    a.color.z = a.color.z + result.z;
-    a.albedo = make_float4(a.albedo.x + al.x, a.albedo.y + al.y, a.albedo.z + al.z, a.albedo.w + al.w);
-    a.normal = make_float4(a.normal.x + nr.x, a.normal.y + nr.y, a.normal.z + nr.z, a.normal.w + nr.w);
+    for (uint32_t i = k << P.shift; i < (k + 1u) << P.shift; ++i) {
+      float4 rs = P.w.res[i];
+      uint32_t flags = __float_as_uint(P.w.ray_d[i].w);
+      v3 result = flush_pending(P, i, flags, mk3(rs.x, rs.y, rs.z));
+      if (flags & F_CACHED) {
+        // the cache's radiance at the vertex the path ended at, through its throughput
+        float4 pr = P.c.pred[i], th = P.w.thr[i];
+        v3 radiance = mk3(fmaxf(pr.x, 0.0f), fmaxf(pr.y, 0.0f), fmaxf(pr.z, 0.0f));
+        result = add3(result, capped(P, mul3(mk3(th.x, th.y, th.z), radiance), true));
+      }
+      if (P.c.enabled) {
+        uint32_t ts = P.c.tslot[i];
+        if (ts != ~0u)
+          emit_records(P.c.tvert, P.c.records, P.w.counters + 7, P.c.rcap, P.c.record_bounces + 1u, ts, result);
+      }
+      float4 al = P.w.alb[i], nr = P.w.nrm[i];
+      a.color.x = a.color.x + result.x;
+      a.color.y = a.color.y + result.y;
+      a.color.z = a.color.z + result.z;
+      a.albedo = make_float4(a.albedo.x + al.x, a.albedo.y + al.y, a.albedo.z + al.z, a.albedo.w + al.w);
+      a.normal = make_float4(a.normal.x + nr.x, a.normal.y + nr.y, a.normal.z + nr.z, a.normal.w + nr.w);
+    }
     accum[pixel] = a;
   }
 }
@@ -1545,8 +1562,21 @@ void launch_light_slots(const Pass& P, cudaStream_t st) {
   }
 }
 
-// Path-state buffers for `capacity` paths and `cap` slots per path.
-void ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap) {
+// Path-state buffers for `capacity` paths and `cap` slots per path: those of
+// one sample a pixel, or (`wide`) those of several, which are an allocation of
+// their own, so that passes captured with either stay valid.  The wide ones
+// take at most a quarter of the memory that is free; false when that does not
+// do.  The counters, the ray totals among them, belong to both.
+bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
+  if (!t.wave_counters) {
+    void* d = nullptr;
+    check(cudaMalloc(&d, 128), "counters");
+    t.owned.push_back(d);
+    check(cudaMemset(d, 0, 128), "counters");
+    t.wave_counters = static_cast<uint32_t*>(d);
+  }
+  void*& buffer = wide ? t.d_wide_wave : t.d_wave;
+  size_t& held = wide ? t.wide_wave_bytes : t.wave_bytes;
   size_t need = 0;
   auto add = [&](size_t bytes) {
     size_t at = (need + 255) & ~size_t(255);
@@ -1558,23 +1588,27 @@ void ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap) {
          o_hit = add(16ull * capacity), o_hitv = add(4ull * capacity), o_sho = add(16ull * capacity * cap),
          o_shd = add(16ull * capacity * cap), o_shc = add(16ull * capacity * cap), o_q0 = add(4ull * capacity),
          o_q1 = add(4ull * capacity), o_sq = add(4ull * capacity * cap), o_act = add(4ull * capacity),
-         o_cnt = add(128), o_keys = add(4ull * capacity), o_sorted = add(4ull * capacity),
+         o_keys = add(4ull * capacity), o_sorted = add(4ull * capacity),
          o_hist = add(4ull * SORT_BINS), o_cursor = add(4ull * SORT_BINS), o_lit = add(4ull * capacity),
          o_surf = add(144ull * capacity), o_rhist = add(4ull * RAY_BINS), o_rcursor = add(4ull * RAY_BINS),
          o_retry = add(4ull * capacity * (cap > 0 ? cap : 1)), o_eretry = add(4ull * capacity),
          o_pick = add(8ull * capacity);
-  if (need > t.wave_bytes) {
-    if (t.d_wave) cudaFree(t.d_wave);
-    t.d_wave = nullptr;
-    t.wave_bytes = 0;
-    trace_forget_graphs(t);  // captured passes name the old buffers
-    check(cudaMalloc(&t.d_wave, need), "wavefront path state");
-    check(cudaMemset(static_cast<char*>(t.d_wave) + o_cnt, 0, 128), "counters");
-    t.wave_bytes = need;
+  if (need > held) {
+    if (wide) {
+      size_t free_bytes = 0, total = 0;
+      check(cudaMemGetInfo(&free_bytes, &total), "wavefront path state");
+      if (need > free_bytes / 4u) return false;
+    }
+    if (buffer) {
+      trace_forget_graphs(t);  // captured passes name the old buffers
+      cudaFree(buffer);
+    }
+    buffer = nullptr;
+    held = 0;
+    check(cudaMalloc(&buffer, need), "wavefront path state");
+    held = need;
   }
-  t.wave_counters = reinterpret_cast<uint32_t*>(static_cast<char*>(t.d_wave) + o_cnt);
-  t.wave_capacity = capacity;
-  char* b = static_cast<char*>(t.d_wave);
+  char* b = static_cast<char*>(buffer);
   Wave& w = *reinterpret_cast<Wave*>(&t.wave_layout);
   w.ray_o = reinterpret_cast<float4*>(b + o_ray_o);
   w.ray_d = reinterpret_cast<float4*>(b + o_ray_d);
@@ -1591,7 +1625,7 @@ void ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap) {
   w.queue[1] = reinterpret_cast<uint32_t*>(b + o_q1);
   w.squeue = reinterpret_cast<uint32_t*>(b + o_sq);
   w.active = reinterpret_cast<uint32_t*>(b + o_act);
-  w.counters = reinterpret_cast<uint32_t*>(b + o_cnt);
+  w.counters = t.wave_counters;
   w.keys = reinterpret_cast<uint32_t*>(b + o_keys);
   w.sorted = reinterpret_cast<uint32_t*>(b + o_sorted);
   w.hist = reinterpret_cast<uint32_t*>(b + o_hist);
@@ -1603,6 +1637,7 @@ void ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap) {
   w.retry = reinterpret_cast<uint32_t*>(b + o_retry);
   w.eretry = reinterpret_cast<uint32_t*>(b + o_eretry);
   w.pick = reinterpret_cast<float2*>(b + o_pick);
+  return true;
 }
 
 // Cache scratch for `pixels` paths: queries, their path indices and
@@ -1711,16 +1746,43 @@ void trace_forget_graphs(pfxt_trace& t) {
 
 static_assert(sizeof(Wave) <= sizeof(((pfxt_trace*)nullptr)->wave_layout), "wave layout storage");
 
-void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed) {
+// Paths a wave may hold by taking several samples of a pixel at once.  One
+// sample of a small frame, or of the few pixels that an adaptive render still
+// samples, leaves most of the GPU idle behind every launch's slowest walks
+// (8 of 32 lanes, ~100 launches a sample).  With the samples one by one, then
+// in waves of 2^21, 2^22 and 2^23 paths (one B200): 512 x 512 at 16 samples
+// 13.3, 4.49, 3.92, 3.92 ms; 1280 x 720 at 16 samples 116, 107.0, 103.3,
+// 103.5; 960 x 540 adaptive to 64 samples 246, 124.8, 114.6, 111.7.  The
+// samples of a pixel are neighbours, so a warp's camera rays stay close.
+constexpr uint32_t WAVE_PATHS = 1u << 22;
+
+// log2 of the samples of `live` pixels that one wave takes, at most `count`.
+static uint32_t wave_shift(uint32_t live, uint32_t count) {
+  uint32_t shift = 0u;
+  while ((2ull << shift) <= count && ((uint64_t)live << (shift + 1u)) <= WAVE_PATHS) ++shift;
+  return shift;
+}
+
+void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed, uint32_t live) {
   if (count == 0) return;
   uint32_t pixels = t.width * t.height;
+  live = std::max(std::min(live, pixels), 1u);
   uint32_t light_slots = 1u + t.shade.looped + (t.shade.tree > 0u ? 1u : 0u);
   uint32_t slots = 2u + light_slots;
   uint32_t cap = std::min(slots, CAP_MAX);
   bool deferred = slots <= CAP_MAX && t.shadow_queue;
-  ensure_wave(t, pixels, cap);
+  // The cache's queries and training paths are counted per sample: one at a time.
+  uint32_t shift = t.cache ? 0u : wave_shift(live, count);
+  uint32_t capacity = shift > 0u ? std::max(pixels, WAVE_PATHS) : pixels;
+  if (shift > 0u && !ensure_wave(t, capacity, cap, true)) {
+    shift = 0u;
+    capacity = pixels;
+  }
+  if (shift == 0u) ensure_wave(t, capacity, cap, false);
   Pass P;
   memset(&P, 0, sizeof(P));
+  P.shift = shift;
+  P.capacity = capacity;
   P.f = t.base;  // the accumulated samples, the count, the seed and the camera travel in P.vars
   P.f.size[2] = 0u;
   P.f.size[3] = 0u;
@@ -1802,7 +1864,7 @@ void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed) {
       cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
       cudaGraphDestroy(graph);
       check(e, "pass graph");
-      if (t.graphs.size() >= 8) {
+      if (t.graphs.size() >= 16) {
         cudaGraphExecDestroy(t.graphs.front().exec);
         t.graphs.erase(t.graphs.begin());
       }
@@ -1855,8 +1917,11 @@ void enqueue_pass(pfxt_trace& t, Pass& P, uint32_t count, bool deferred, uint32_
   // (its own work counter, retry list and queue count), and the bounce joins
   // it before shading.
   const bool ahead = TRACE_AHEAD && deferred;
-  for (uint32_t sample = 0; sample < count; ++sample) {
+  const uint32_t widest = P.shift;
+  for (uint32_t sample = 0; sample < count; sample += 1u << P.shift) {
     P.sample = sample;
+    P.shift = widest;
+    while ((1u << P.shift) > count - sample) --P.shift;
     if (P.c.enabled) k_cache_begin<<<1, 32, 0, st>>>(P);
     k_gen<<<g.flat, 256, 0, st>>>(P);
     k_seed_counts<<<1, 32, 0, st>>>(P);
@@ -2027,7 +2092,7 @@ void trace_sample_adaptive(pfxt_trace& t, const pfxt_adaptive& a, uint32_t seed,
     check(cudaMemsetAsync(t.d_snaps, 0, (size_t)pixels * 32, st), "snapshots");
   }
   Grids& g = grids();
-  uint32_t n = 0;
+  uint32_t n = 0, live = pixels;  // pixels that still sample
   for (const pfxt_round& r : reached) {
     if (rounds && n < cap) rounds[n] = r;
     ++n;
@@ -2038,11 +2103,11 @@ void trace_sample_adaptive(pfxt_trace& t, const pfxt_adaptive& a, uint32_t seed,
     if (keeping && keeping->due) {
       // one sample at a time, offering a checkpoint after each (adaptive.rs:258-277)
       for (uint32_t s = 0; s < count; ++s) {
-        trace_sample(t, 1u, seed);
+        trace_sample(t, 1u, seed, live);
         if (keeping->due(t.samples)) keeping->keep(reached);
       }
     } else {
-      trace_sample(t, count, seed);
+      trace_sample(t, count, seed, live);
     }
     check(cudaMemsetAsync(t.d_running, 0, 4, st), "running count");
     k_measure<<<g.flat, 256, 0, st>>>(t.d_accum, t.d_snaps, t.width, t.height);
@@ -2052,6 +2117,7 @@ void trace_sample_adaptive(pfxt_trace& t, const pfxt_adaptive& a, uint32_t seed,
     check(cudaMemcpyAsync(&running, t.d_running, 4, cudaMemcpyDeviceToHost, st), "running count");
     check(cudaStreamSynchronize(st), "convergence");
     uint64_t active = step > 0 ? (uint64_t)running : (uint64_t)pixels;
+    live = (uint32_t)active;
     pfxt_round round{target, 0u, active};
     reached.push_back(round);
     if (rounds && n < cap) rounds[n] = round;

@@ -116,10 +116,11 @@ struct pfxt_trace {
   // wavefront scratch (allocated on first use)
   void* d_wave = nullptr;
   size_t wave_bytes = 0;
-  uint32_t wave_capacity = 0;
-  alignas(16) unsigned char wave_layout[256];  // pointers into d_wave (tracer.cu)
+  void* d_wide_wave = nullptr;  // of waves of several samples a pixel
+  size_t wide_wave_bytes = 0;
+  alignas(16) unsigned char wave_layout[256];  // pointers into one of them (tracer.cu)
   uint32_t light_rows = 0;                     // rows of the light buffer (lights + tree)
-  uint32_t* wave_counters = nullptr;           // queue counters and ray totals inside d_wave
+  uint32_t* wave_counters = nullptr;           // queue counters and ray totals
   uint8_t* d_mask = nullptr;                   // optional per-pixel mask of the pixels to sample
   bool sort_shading = true;                    // group the shade queue by material every bounce
   uint32_t trace_threads = 128;                // threads per block of the traversal kernels (64, 128, 256)
@@ -165,7 +166,9 @@ void trace_release(pfxt_trace& t);
 void trace_set_camera(pfxt_trace& t, const pfxt_camera& c);
 void trace_set_lens(pfxt_trace& t, const float lens[4]);
 void trace_set_window(pfxt_trace& t, const uint32_t full[2], const uint32_t origin[2]);
-void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed);
+// `live`: at most so many pixels still sample (an adaptive render's running
+// count), which decides how many samples of a pixel one wave takes.
+void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed, uint32_t live = ~0u);
 // The light rows' cone trigonometry (ShadeView::light_trig), once per tracer.
 void light_trig_init(pfxt_trace& t);
 // Drops the captured passes (their buffers or launch parameters changed).

@@ -248,6 +248,8 @@ void trace_release(pfxt_trace& t) {
   t.owned.clear();
   if (t.d_wave) cudaFree(t.d_wave);
   t.d_wave = nullptr;
+  if (t.d_wide_wave) cudaFree(t.d_wide_wave);
+  t.d_wide_wave = nullptr;
   if (t.d_stage) cudaFree(t.d_stage);
   t.d_stage = nullptr;
   if (t.d_cache_scratch) cudaFree(t.d_cache_scratch);
