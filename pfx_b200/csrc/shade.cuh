@@ -112,7 +112,7 @@ SH_SMALL float4 sobol4(const ShadeView& v, const Specialise& sp, const Rng& r, u
   uint32_t mask = L - 1u;
   uint32_t shuffled = brev_(reversed_bit_owen(brev_(r.y), hash_wang_seeded(dim, seed)));
   uint32_t sample = (r.y & ~mask) | (shuffled & mask);
-  uint32_t index = (pattern * L + sample) % (L * 256u);
+  uint32_t index = (pattern * L + sample) & (L * 256u - 1u);  // L is a power of two
   float4 t = __ldg(v.sobol + index);
   float s0 = (float)hash_wang_seeded(dim, seed) * 2.3283064e-10f;
   float s1 = (float)hash_wang_seeded(dim, seed ^ 0xca0e1151u) * 2.3283064e-10f;
@@ -120,6 +120,16 @@ SH_SMALL float4 sobol4(const ShadeView& v, const Specialise& sp, const Rng& r, u
   float s3 = (float)hash_wang_seeded(dim, seed ^ 0x99634d1du) * 2.3283064e-10f;
   return make_float4(fmin_(fract_(t.x + s0), 0.99999994f), fmin_(fract_(t.y + s1), 0.99999994f),
                      fmin_(fract_(t.z + s2), 0.99999994f), fmin_(fract_(t.w + s3), 0.99999994f));
+}
+// sobol4's third component alone.
+__device__ __forceinline__ float sobol_z(const ShadeView& v, const Specialise& sp, const Rng& r, uint32_t dimension) {
+  const uint32_t L = sp.sobol_length, seed = r.x, dim = r.z + dimension, mask = L - 1u;
+  const uint32_t pattern = hash_shuffle_256(dim, seed);
+  const uint32_t shuffled = brev_(reversed_bit_owen(brev_(r.y), hash_wang_seeded(dim, seed)));
+  const uint32_t sample = (r.y & ~mask) | (shuffled & mask);
+  const uint32_t index = (pattern * L + sample) & (L * 256u - 1u);
+  const float t = __ldg(reinterpret_cast<const float*>(v.sobol + index) + 2);
+  return fmin_(fract_(t + (float)hash_wang_seeded(dim, seed ^ 0xbf604c5au) * 2.3283064e-10f), 0.99999994f);
 }
 __device__ __forceinline__ float rnd(const Specialise& sp, uint32_t& state, float value) {
   if (sp.sobol) return value;
@@ -622,11 +632,8 @@ __device__ __forceinline__ float sin_from_cos(float c) { return sqrtf(fmax_(1.0f
 
 // tree_importance (lights.wgsl:204-237) -> (max, min)
 // trig = (cos theta_o, sin theta_o, cos(theta_o + theta_e), cos(theta_e - theta_o)).
-// The light-tree functions are written once as inline bodies (`*_b`); IN
-// selects whether a body calls the next ones inline (the descent kernel) or
-// through their out-of-line copies (the kernels that keep them out of line).
-__device__ __forceinline__ float2 tree_importance_b(v3 n, v3 to, float cos_u, v3 axis, float theta_o, float theta_e,
-                                                    float far, float near, float energy, float4 trig) {
+SH_SMALL float2 tree_importance(v3 n, v3 to, float cos_u, v3 axis, float theta_o, float theta_e, float far,
+                                float near, float energy, float4 trig) {
   float sin_u = sin_from_cos(cos_u);
   float cos_i = dot3(to, n);
   float sin_i = sin_from_cos(cos_i);
@@ -657,18 +664,7 @@ __device__ __forceinline__ float2 tree_importance_b(v3 n, v3 to, float cos_u, v3
   float cos_max_out = cos_t_plus_u * cos_o - sin_from_cos(cos_t_plus_u) * sin_o;
   return make_float2(most, abs_(cos_max_i * energy * cos_max_out / (far * far)));
 }
-SH_SMALL float2 tree_importance(v3 n, v3 to, float cos_u, v3 axis, float theta_o, float theta_e, float far,
-                                float near, float energy, float4 trig) {
-  return tree_importance_b(n, to, cos_u, axis, theta_o, theta_e, far, near, energy, trig);
-}
-template <bool IN>
-__device__ __forceinline__ float2 tree_importance_to(v3 n, v3 to, float cos_u, v3 axis, float theta_o, float theta_e,
-                                                     float far, float near, float energy, float4 trig) {
-  if constexpr (IN) return tree_importance_b(n, to, cos_u, axis, theta_o, theta_e, far, near, energy, trig);
-  return tree_importance(n, to, cos_u, axis, theta_o, theta_e, far, near, energy, trig);
-}
-template <bool IN>
-__device__ __forceinline__ float2 node_importance_b(const LightRow& node, float4 trig, v3 p, v3 n) {
+SH_SMALL float2 node_importance(const LightRow& node, float4 trig, v3 p, v3 n) {
   v3 lo = f3of(node.a), hi = f3of(node.b);
   v3 centroid = scl3(add3(lo, hi), 0.5f);
   v3 extent = sub3(hi, centroid);
@@ -680,15 +676,11 @@ __device__ __forceinline__ float2 node_importance_b(const LightRow& node, float4
   float cos_u = -1.0f;
   if (reach * reach > radius2) cos_u = sqrtf(fmax_(1.0f - radius2 / (reach * reach), 0.0f));
   float distance = fmax_(fmax_(0.5f * sqrtf(radius2), reach), 1e-6f);
-  return tree_importance_to<IN>(n, divs3(to, fmax_(reach, 1e-30f)), cos_u, f3of(node.c), node.c.w, node.d.x,
+  return tree_importance(n, divs3(to, fmax_(reach, 1e-30f)), cos_u, f3of(node.c), node.c.w, node.d.x,
                                 distance, distance, node.a.w, trig);
 }
-SH_SMALL float2 node_importance(const LightRow& node, float4 trig, v3 p, v3 n) {
-  return node_importance_b<false>(node, trig, p, n);
-}
 // trig: the light's RowTrig::light.
-template <bool IN>
-__device__ __forceinline__ float2 emitter_importance_b(const LightRow& light, float4 trig, v3 p, v3 n) {
+SH_SMALL float2 emitter_importance(const LightRow& light, float4 trig, v3 p, v3 n) {
   v3 to = sub3(f3of(light.a), p);
   float near = length3(to);
   if (near >= light.b.w || near <= 1e-6f) return make_float2(0.0f, 0.0f);
@@ -703,26 +695,16 @@ __device__ __forceinline__ float2 emitter_importance_b(const LightRow& light, fl
     float cos_min_out = cos_(fmax_(0.0f, acos_(clamp_(dot3(f3of(light.c), neg3(toward)), -1.0f, 1.0f)) - acos_(cos_u)));
     float along = clamp_(cos_min_out * light.d.x + light.d.y, 0.0f, 1.0f);
     energy = energy * (along * along);
-    return tree_importance_to<IN>(n, toward, cos_u, f3of(light.c), 0.0f, theta_e, far, near, energy, cones);
+    return tree_importance(n, toward, cos_u, f3of(light.c), 0.0f, theta_e, far, near, energy, cones);
   }
-  return tree_importance_to<IN>(n, toward, cos_u, neg3(toward), 0.0f, trig.x, far, near, energy, cones);
+  return tree_importance(n, toward, cos_u, neg3(toward), 0.0f, trig.x, far, near, energy, cones);
 }
-SH_SMALL float2 emitter_importance(const LightRow& light, float4 trig, v3 p, v3 n) {
-  return emitter_importance_b<false>(light, trig, p, n);
-}
-template <bool IN>
-__device__ __forceinline__ float2 emitter_importance_to(const LightRow& light, float4 trig, v3 p, v3 n) {
-  if constexpr (IN) return emitter_importance_b<true>(light, trig, p, n);
-  return emitter_importance(light, trig, p, n);
-}
-template <bool IN>
 __device__ __forceinline__ float2 child_importance(const ShadeView& v, uint32_t row, v3 p, v3 n) {
   LightRow node = load_light(v, row);
   if (f2u(node.d.y) == 1u) {
     uint32_t light = f2u(node.d.z);
-    return emitter_importance_to<IN>(load_light(v, light), load_trig(v, light).light, p, n);
+    return emitter_importance(load_light(v, light), load_trig(v, light).light, p, n);
   }
-  if constexpr (IN) return node_importance_b<true>(node, load_trig(v, row).node, p, n);
   return node_importance(node, load_trig(v, row).node, p, n);
 }
 
@@ -730,9 +712,8 @@ __device__ __forceinline__ float2 child_importance(const ShadeView& v, uint32_t 
 // leaf holds one light whose importance the descent has already evaluated
 // (child_importance of that leaf: emitter_importance of the same light row
 // at the same point), passed as `known` instead of being evaluated again.
-template <bool IN>
-__device__ __forceinline__ float2 tree_leaf_b(const ShadeView& v, uint32_t first, uint32_t count, v3 p, v3 n,
-                                              float start, float2 known, bool use_known) {
+SH_TREE float2 tree_leaf(const ShadeView& v, uint32_t first, uint32_t count, v3 p, v3 n, float start, float2 known,
+                         bool use_known) {
   float rand = start;
   bool sample_max = rand > 0.5f;
   if (count > 1u) rand = rand * 2.0f - (sample_max ? 1.0f : 0.0f);
@@ -743,7 +724,7 @@ __device__ __forceinline__ float2 tree_leaf_b(const ShadeView& v, uint32_t first
     int32_t index = (int32_t)(first + i);
     float2 importance = (use_known && i == 0u)
                             ? known
-                            : emitter_importance_to<IN>(load_light(v, first + i), load_trig(v, first + i).light, p, n);
+                            : emitter_importance(load_light(v, first + i), load_trig(v, first + i).light, p, n);
     float weight = sample_max ? importance.x : importance.y;
     float other = sample_max ? importance.y : importance.x;
     if (weight > 0.0f) {
@@ -802,7 +783,7 @@ __device__ __forceinline__ float2 tree_leaf_b(const ShadeView& v, uint32_t first
       total_min = valid;
       chosen_max = (use_known && (uint32_t)selected == first)
                        ? known.x
-                       : emitter_importance_to<IN>(load_light(v, (uint32_t)selected),
+                       : emitter_importance(load_light(v, (uint32_t)selected),
                                                    load_trig(v, (uint32_t)selected).light, p, n).x;
     }
   }
@@ -811,13 +792,7 @@ __device__ __forceinline__ float2 tree_leaf_b(const ShadeView& v, uint32_t first
 
 // tree_pick (lights.wgsl:350-386): (light row, pmf).  The descent is bounded
 // by the number of tree rows; a malformed tree ends the descent with pmf 0.
-SH_TREE float2 tree_leaf(const ShadeView& v, uint32_t first, uint32_t count, v3 p, v3 n, float start, float2 known,
-                         bool use_known) {
-  return tree_leaf_b<false>(v, first, count, p, n, start, known, use_known);
-}
-template <bool IN>
-__device__ __forceinline__ float2 tree_pick_b(const ShadeView& v, uint32_t rows, v3 p, v3 n, float start,
-                                              uint32_t* leaf_row) {
+SH_TREE float2 tree_pick(const ShadeView& v, uint32_t rows, v3 p, v3 n, float start, uint32_t* leaf_row) {
   uint32_t at = f2u((float)v.looped + (float)v.tree);
   float rand = start;
   float pdf = 1.0f;
@@ -830,15 +805,14 @@ __device__ __forceinline__ float2 tree_pick_b(const ShadeView& v, uint32_t rows,
     if (count > 0u) {
       if (leaf_row) *leaf_row = at;
       const bool use_known = evaluated && count == 1u;
-      float2 leaf = IN ? tree_leaf_b<true>(v, f2u(node.d.z), count, p, n, rand, known, use_known)
-                       : tree_leaf(v, f2u(node.d.z), count, p, n, rand, known, use_known);
+      float2 leaf = tree_leaf(v, f2u(node.d.z), count, p, n, rand, known, use_known);
       return make_float2(leaf.x, leaf.y * pdf);
     }
     uint32_t left = at + 1u;
     uint32_t right = f2u(node.d.z);
     if (right >= rows) break;
-    float2 l = child_importance<IN>(v, left, p, n);
-    float2 r = child_importance<IN>(v, right, p, n);
+    float2 l = child_importance(v, left, p, n);
+    float2 r = child_importance(v, right, p, n);
     float total_max = l.x + r.x;
     if (total_max == 0.0f) return make_float2(0.0f, 0.0f);
     float total_min = l.y + r.y;
@@ -863,8 +837,222 @@ __device__ __forceinline__ float2 tree_pick_b(const ShadeView& v, uint32_t rows,
   }
   return make_float2(0.0f, 0.0f);
 }
-SH_TREE float2 tree_pick(const ShadeView& v, uint32_t rows, v3 p, v3 n, float start, uint32_t* leaf_row) {
-  return tree_pick_b<false>(v, rows, p, n, start, leaf_row);
+
+// ------------------------------------------------------------ the descent on its own rows
+// A light-tree row as the descent kernel reads it: what node_importance and
+// emitter_importance work out from the row alone, by the same expressions,
+// once per tracer (k_pick_rows).  A leaf of one light holds that light's.
+enum PickKind : uint32_t { PICK_NODE = 0u, PICK_POINT = 1u, PICK_SPOT = 2u };
+struct alignas(128) PickRow {
+  // node: centroid, |hi - centroid|^2; light: position, radius
+  float center[3], radius2;
+  // node: |hi - centroid| per axis, half the box's half diagonal; light: axis, radius^2
+  float extent[3], half;
+  // node: the box; light: lo[0], lo[1] = the spot's scale and offset, lo[2] = range
+  float lo[3], reach2;  // reach2: the least squared distance whose root is at least the range
+  float hi[3], energy;
+  // cos theta_o, sin theta_o, cos(theta_o + theta_e), cos(theta_e - theta_o)
+  float trig[4];
+  float axis[3];
+  uint32_t link;   // node: the right child's row; leaf: its first light
+  uint32_t count;  // lights of a leaf, 0 for an inner node
+  uint32_t kind;   // of this row as a child (PickKind)
+  uint32_t wide;   // theta_o + theta_e > pi
+  uint32_t narrow; // theta_e - theta_o < 0
+  float pad[4];
+};
+static_assert(sizeof(PickRow) == 128, "PickRow");
+
+// x / m per component, correctly rounded: Markstein's correction (quotient() in
+// traverse.cuh) from one reciprocal where nothing can underflow, else the
+// divisions themselves.  |x| <= m (1 + 2^-20), as for a vector and its length.
+__device__ __forceinline__ v3 over_length(v3 x, float m) {
+  const float least = fminf(fminf(fabsf(x.x), fabsf(x.y)), fabsf(x.z));
+  if (!(least >= 0x1p-60f && m <= 0x1p+60f)) return divs3(x, m);
+  const float r = 1.0f / m;
+  const float qx = x.x * r, qy = x.y * r, qz = x.z * r;
+  return mk3(fmaf(fmaf(-qx, m, x.x), r, qx), fmaf(fmaf(-qy, m, x.y), r, qy), fmaf(fmaf(-qz, m, x.z), r, qz));
+}
+// fmax_(1 - c^2, 0): no signed zero reaches the comparison, so the plain maximum.
+__device__ __forceinline__ float sin_of(float c) { return sqrtf(fmaxf(1.0f - c * c, 0.0f)); }
+
+// child_importance (max, min) of row `row`.  The kinds differ in what they
+// hand to tree_importance, which all lanes of a warp then run together.
+__device__ __forceinline__ float2 pick_importance(const PickRow* __restrict__ rows, uint32_t row, v3 p, v3 n) {
+  const float4* q = reinterpret_cast<const float4*>(rows + row);
+  const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2);
+  const float4 trig = __ldg(q + 4);
+  const float4 q5 = __ldg(q + 5);
+  const uint4 q6 = __ldg(reinterpret_cast<const uint4*>(q + 6));
+  const v3 to = sub3(f3of(q0), p);
+  float cos_u, near, far, energy;
+  v3 toward, axis = f3of(q5);
+  bool live;
+  if (q6.y == PICK_NODE) {
+    const float4 q3 = __ldg(q + 3);
+    energy = q3.w;
+    const v3 off = sub3(p, mk3(fminf(fmaxf(p.x, q2.x), q3.x), fminf(fmaxf(p.y, q2.y), q3.y),
+                               fminf(fmaxf(p.z, q2.z), q3.z)));
+    live = !(dot3(n, to) + dot3(mk3(fabsf(n.x), fabsf(n.y), fabsf(n.z)), f3of(q1)) <= 0.0f) &&
+           !(dot3(off, off) >= q2.w);
+    if (!live) return make_float2(0.0f, 0.0f);
+    const float reach = length3(to), square = reach * reach;
+    cos_u = square > q0.w ? sqrtf(fmaxf(1.0f - q0.w / square, 0.0f)) : -1.0f;
+    near = far = fmaxf(fmaxf(q1.w, reach), 1e-6f);
+    toward = over_length(to, fmaxf(reach, 1e-30f));
+  } else {
+    near = length3(to);
+    live = !(near >= q2.z || near <= 1e-6f);
+    if (!live) return make_float2(0.0f, 0.0f);
+    toward = over_length(to, near);
+    far = sqrtf(q1.w + near * near);
+    cos_u = near / far;
+    energy = __ldg(reinterpret_cast<const float*>(q + 3) + 3);
+    if (q6.y == PICK_SPOT) {
+      const float cos_min_out = cos_(fmaxf(0.0f, acos_(fminf(fmaxf(dot3(axis, neg3(toward)), -1.0f), 1.0f)) -
+                                                     acos_(cos_u)));
+      const float along = fminf(fmaxf(cos_min_out * q2.x + q2.y, 0.0f), 1.0f);
+      energy = energy * (along * along);
+    } else {
+      axis = neg3(toward);
+    }
+  }
+  // tree_importance
+  const float sin_u = sin_of(cos_u);
+  const float cos_i = dot3(toward, n);
+  const float sin_i = sin_of(cos_i);
+  const float cos_min_i = cos_i >= cos_u ? 1.0f : cos_i * cos_u + sin_i * sin_u;
+  if (cos_min_i < 0.0f) return make_float2(0.0f, 0.0f);
+  const float cos_max_i = fmaxf(cos_i * cos_u - sin_i * sin_u, 0.0f);
+  float cos_t = 1.0f, sin_t = 0.0f;
+  const v3 nt = neg3(toward);
+  if (axis.x != nt.x || axis.y != nt.y || axis.z != nt.z) {
+    cos_t = dot3(axis, nt);
+    sin_t = sin_of(cos_t);
+  }
+  const float cos_t_minus_u = cos_t * cos_u + sin_t * sin_u;
+  float cos_min_out;
+  if (cos_t >= cos_u || cos_t_minus_u >= trig.x) {
+    cos_min_out = 1.0f;
+  } else if (q6.z != 0u || cos_t_minus_u > trig.z) {
+    cos_min_out = cos_t_minus_u * trig.x + sin_of(cos_t_minus_u) * trig.y;
+  } else {
+    return make_float2(0.0f, 0.0f);
+  }
+  const float most = fabsf(cos_min_i * energy * cos_min_out / (near * near));
+  const float cos_t_plus_u = cos_t * cos_u - sin_t * sin_u;
+  if (q6.w != 0u || cos_t < 0.0f || cos_u < 0.0f || cos_t_plus_u < trig.w) return make_float2(most, 0.0f);
+  const float cos_max_out = cos_t_plus_u * trig.x - sin_of(cos_t_plus_u) * trig.y;
+  return make_float2(most, fabsf(cos_max_i * energy * cos_max_out / (far * far)));
+}
+
+// tree_pick on the PickRows: the same values bit for bit.
+__device__ __forceinline__ float2 tree_pick_rows(const ShadeView& v, uint32_t rows, v3 p, v3 n, float start) {
+  const PickRow* __restrict__ table = v.pick_rows;
+  uint32_t at = f2u((float)v.looped + (float)v.tree);
+  float rand = start, pdf = 1.0f;
+  float2 known = make_float2(0.0f, 0.0f);
+  bool evaluated = false;
+  for (uint32_t guard = 0u; guard < rows; ++guard) {
+    if (at >= rows) break;
+    const uint32_t count = __ldg(&table[at].count), link = __ldg(&table[at].link);
+    if (count > 0u) {
+      if (evaluated && count == 1u) {
+        // tree_leaf of one light whose importance is known: x / x and y / y
+        // (1 for y = 0) whichever of the two the random number picks
+        if (!(known.x > 0.0f)) return make_float2(0.0f, 0.0f);
+        const float finite = known.x < INFINITY && known.y < INFINITY
+                                 ? 1.0f
+                                 : 0.5f * (known.x / known.x + (known.y == 0.0f ? 1.0f : known.y / known.y));
+        return make_float2((float)(int32_t)link, finite * pdf);
+      }
+      const float2 leaf = tree_leaf(v, link, count, p, n, rand, known, false);
+      return make_float2(leaf.x, leaf.y * pdf);
+    }
+    const uint32_t left = at + 1u;
+    if (link >= rows) break;
+    float2 l = make_float2(0.0f, 0.0f), r = l;
+#pragma unroll 1
+    for (uint32_t c = 0u; c < 2u; ++c) {  // one body for both children: the kernel is bound by issue and code
+      const float2 w = pick_importance(table, c ? link : left, p, n);
+      if (c == 0u)
+        l = w;
+      else
+        r = w;
+    }
+    const float total_max = l.x + r.x;
+    if (total_max == 0.0f) return make_float2(0.0f, 0.0f);
+    const float total_min = l.y + r.y;
+    float probability_min = 0.5f * ((l.x > 0.0f ? 1.0f : 0.0f) + (r.x == 0.0f ? 1.0f : 0.0f));
+    if (total_min > 0.0f) probability_min = l.y / total_min;
+    const float left_probability = 0.5f * (l.x / total_max + probability_min);
+    const float right_weight = 1.0f - left_probability;
+    at = left;
+    if (right_weight > 0.0f) {
+      const float thresh = right_weight / (left_probability + right_weight);
+      const bool right = rand <= thresh;
+      if (right) at = link;
+      rand = (right ? rand : rand - thresh) / (right ? thresh : 1.0f - thresh);
+      rand = fminf(fmaxf(rand, 0.0f), 1.0f);
+    }
+    pdf = pdf * (at == left ? left_probability : 1.0f - left_probability);
+    known = at == left ? l : r;
+    evaluated = true;
+  }
+  return make_float2(0.0f, 0.0f);
+}
+
+// The PickRow of row i (0 <= i < rows).
+__device__ __forceinline__ PickRow make_pick_row(const ShadeView& v, uint32_t rows, uint32_t i) {
+  PickRow out;
+  const LightRow node = load_light(v, i);
+  const RowTrig trig = load_trig(v, i);
+  out.count = f2u(node.d.y);
+  out.link = f2u(node.d.z);
+  out.pad[0] = out.pad[1] = out.pad[2] = out.pad[3] = 0.0f;
+  const bool leaf = out.count == 1u && out.link < rows;
+  if (!leaf) {
+    const v3 lo = f3of(node.a), hi = f3of(node.b);
+    const v3 centroid = scl3(add3(lo, hi), 0.5f);
+    const v3 extent = sub3(hi, centroid), size = abs3(extent);
+    out.center[0] = centroid.x, out.center[1] = centroid.y, out.center[2] = centroid.z;
+    out.radius2 = dot3(extent, extent);
+    out.extent[0] = size.x, out.extent[1] = size.y, out.extent[2] = size.z;
+    out.half = 0.5f * sqrtf(out.radius2);
+    out.lo[0] = lo.x, out.lo[1] = lo.y, out.lo[2] = lo.z;
+    out.hi[0] = hi.x, out.hi[1] = hi.y, out.hi[2] = hi.z;
+    // the least s with sqrtf(s) >= the range (sqrtf is monotone)
+    const float range = node.b.w;
+    float s = range <= 0.0f ? 0.0f : range * range;
+    if (range > 0.0f) {
+      for (int k = 0; k < 8 && s > 0.0f && sqrtf(bits2f(f2bits(s) - 1u)) >= range; ++k) s = bits2f(f2bits(s) - 1u);
+      for (int k = 0; k < 8 && sqrtf(s) < range; ++k) s = bits2f(f2bits(s) + 1u);
+    }
+    out.reach2 = s;
+    out.energy = node.a.w;
+    out.trig[0] = trig.node.x, out.trig[1] = trig.node.y, out.trig[2] = trig.node.z, out.trig[3] = trig.node.w;
+    out.axis[0] = node.c.x, out.axis[1] = node.c.y, out.axis[2] = node.c.z;
+    out.kind = PICK_NODE;
+    out.wide = node.c.w + node.d.x > SH_PI ? 1u : 0u;
+    out.narrow = node.d.x - node.c.w < 0.0f ? 1u : 0u;
+    return out;
+  }
+  const LightRow light = load_light(v, out.link);
+  const float4 t = load_trig(v, out.link).light;
+  out.center[0] = light.a.x, out.center[1] = light.a.y, out.center[2] = light.a.z;
+  out.radius2 = light.c.w;
+  out.extent[0] = out.extent[1] = out.extent[2] = 0.0f;
+  out.half = light.c.w * light.c.w;
+  out.lo[0] = light.d.x, out.lo[1] = light.d.y, out.lo[2] = light.b.w;
+  out.reach2 = 0.0f;
+  out.hi[0] = out.hi[1] = out.hi[2] = 0.0f;
+  out.energy = (light.b.x + light.b.y + light.b.z) / 3.0f;
+  out.trig[0] = t.z, out.trig[1] = t.w, out.trig[2] = t.y, out.trig[3] = t.y;
+  out.axis[0] = light.c.x, out.axis[1] = light.c.y, out.axis[2] = light.c.z;
+  out.kind = f2u(light.a.w) == 1u ? PICK_SPOT : PICK_POINT;
+  out.wide = 0.0f + t.x > SH_PI ? 1u : 0u;
+  out.narrow = t.x - 0.0f < 0.0f ? 1u : 0u;
+  return out;
 }
 
 // ------------------------------------------------------------ emitters

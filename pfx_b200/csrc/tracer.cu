@@ -1164,17 +1164,8 @@ constexpr int SLOT_SUN = 0, SLOT_SKY = 1, SLOT_EMITTER = 2, SLOT_LOOPED = 3, SLO
 #define SLOT_MIN_BLOCKS 8
 #endif
 #ifndef PICK_MIN_BLOCKS
-#define PICK_MIN_BLOCKS 8
+#define PICK_MIN_BLOCKS 10
 #endif
-// Whether the descent kernel runs the light-tree functions inline or through their out-of-line copies.
-// Plain 4K pass: out of line at 12 blocks per SM 93.1 ms, at 8 blocks 92.5; inline at 12, 10 and 8
-// blocks 102.8, 104.8 and 108.1 ms (more code, fewer lanes per instruction).  Later, with the one-light
-// leaves reusing the descent's importance: 8 blocks (64 registers) 91.5 ms, 6 blocks (72 registers, no
-// spills) 91.7, 4 blocks 91.8.
-#ifndef PICK_INLINE
-#define PICK_INLINE false
-#endif
-
 __device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i) {
   const uint32_t pixel = __float_as_uint(reinterpret_cast<const float*>(P.w.res + i)[3]);
   uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
@@ -1182,7 +1173,14 @@ __device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i) {
 }
 
 // The light tree's descent for every scattering path (slot k of tree_pick's
-// caller in k_shade_lights): the pick (light row, pmf) at P.w.pick[qi].
+// caller in k_shade_lights): the pick (light row, pmf) at P.w.pick[qi].  Bound
+// by issue slots (73 % busy).  With the reference's rows through out-of-line
+// helpers a 100k-triangle room's 3.6 M descents took 1687 us, 12,000
+// instructions a warp at 17 of 32 lanes, with 290 M sectors of local memory;
+// on PickRows (what depends on the row alone worked out once, one tail for all
+// kinds of children, one loop body for both children) 1038 us and 7,200.
+// Blocks of 128 per SM: 6, 8, 10 and 12 gave a 1280 x 720 frame at 16 samples
+// 91.1, 90.6, 90.2 and 96.4 ms.
 __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const __grid_constant__ Pass P, uint32_t k) {
   const uint32_t n = P.w.counters[12];
   const Specialise& sp = P.sp;
@@ -1194,13 +1192,12 @@ __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const _
     uint32_t state = __float_as_uint(reinterpret_cast<const float*>(P.w.thr + i)[3]);
     float start;
     if (sp.sobol) {
-      start = sobol4(V, sp, slot_rng(P, i), light_dim(k)).z;
+      start = sobol_z(V, sp, slot_rng(P, i), light_dim(k));
     } else {
       start = random01(state);
       reinterpret_cast<float*>(P.w.thr + i)[3] = __uint_as_float(state);
     }
-    P.w.pick[qi] = tree_pick_b<PICK_INLINE>(V, P.light_rows, mk3(g0.x, g0.y, g0.z), mk3(g1.x, g1.y, g1.z), start,
-                                           nullptr);
+    P.w.pick[qi] = tree_pick_rows(V, P.light_rows, mk3(g0.x, g0.y, g0.z), mk3(g1.x, g1.y, g1.z), start);
   }
 }
 
@@ -1724,16 +1721,26 @@ __global__ void k_light_trig(const __grid_constant__ ShadeView V, uint32_t rows,
     out[2u * i + 1u] = make_float4(cone, cos_(cone), cos_(0.0f), sin_(0.0f));
   }
 }
+__global__ void k_pick_rows(const __grid_constant__ ShadeView V, uint32_t rows, PickRow* __restrict__ out) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x)
+    out[i] = make_pick_row(V, rows, i);
+}
 }  // namespace
 
 void light_trig_init(pfxt_trace& t) {
   uint32_t rows = std::max<uint32_t>(t.light_rows, 1u);
+  void* picks = nullptr;
+  check(cudaMalloc(&picks, (size_t)rows * sizeof(PickRow)), "light-tree rows");
+  t.owned.push_back(picks);
+  t.shade.pick_rows = static_cast<const PickRow*>(picks);
   void* d = nullptr;
   check(cudaMalloc(&d, (size_t)rows * 32u), "light-row trigonometry");
   t.owned.push_back(d);
   t.shade.light_trig = static_cast<const float4*>(d);
   if (t.light_rows) {
     k_light_trig<<<(t.light_rows + 127u) / 128u, 128, 0, t.stream>>>(t.shade, t.light_rows, static_cast<float4*>(d));
+    k_pick_rows<<<(t.light_rows + 127u) / 128u, 128, 0, t.stream>>>(t.shade, t.light_rows,
+                                                                    static_cast<PickRow*>(picks));
     check(cudaGetLastError(), "light-row trigonometry");
   }
   check(cudaStreamSynchronize(t.stream), "light-row trigonometry");

@@ -52,6 +52,7 @@ struct ShadeView {
   const float* __restrict__ emitter_cdf;
   const GpuLight* __restrict__ lights;
   const float4* __restrict__ light_trig;  // 2 float4 per light row: its cones' trigonometry (shade.cuh RowTrig)
+  const struct PickRow* __restrict__ pick_rows;  // the light rows as the tree's descent reads them (shade.cuh)
   const float* __restrict__ sky_rows;
   const float* __restrict__ sky_columns;
   const float4* __restrict__ sobol;
