@@ -394,7 +394,7 @@ int pfxt_finish_tops(pfxt_trace* trace, const pfxt_buffers* buffers);
  * computes.  No counterpart in the reference (wgpu sizes its own dispatches). */
 typedef struct pfxt_tuning {
   uint32_t trace_threads; /* threads per block of the persistent traversal kernels: 64, 128 or 256 (128) */
-  uint32_t sort_shading;  /* sort the shade queue by hit material every bounce (1) */
+  uint32_t sort_shading;  /* sort the shade queue by hit material every bounce (0) */
   uint32_t graphs;        /* replay each pass from a captured CUDA graph (1) */
   uint32_t split_shade;   /* shade a bounce in three kernels (hit, light slots, BSDF) instead of one (1) */
   uint32_t sort_rays;     /* sort the rays of every bounce after the first by direction and origin (0) */

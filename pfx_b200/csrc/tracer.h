@@ -123,7 +123,13 @@ struct pfxt_trace {
   uint32_t light_rows = 0;                     // rows of the light buffer (lights + tree)
   uint32_t* wave_counters = nullptr;           // queue counters and ray totals
   uint8_t* d_mask = nullptr;                   // optional per-pixel mask of the pixels to sample
-  bool sort_shading = true;                    // group the shade queue by material every bounce
+  // Group the shade queue by material every bounce.  It was laid down for the
+  // fused shade kernel, whose warps run one BSDF's code then (270 -> 247 ms a
+  // 4K pass); the split kernels lose more from gathering paths out of order:
+  // sorted and unsorted, 1280 x 720 at 16 samples 90.0 and 77.9 ms, the 4K
+  // pass 81.7 and 70.7, a 320 x 180 preview 1.52 and 1.40, 512 x 512 at 16
+  // samples 4.05 and 3.87, a cached 1080p pass 9.81 and 9.51.
+  bool sort_shading = false;
   uint32_t trace_threads = 128;                // threads per block of the traversal kernels (64, 128, 256)
   bool split_shade = true;                     // shade in three kernels (hit, lights, BSDF) or one
   bool sort_rays = false;                      // group the extend queue of later bounces by ray
