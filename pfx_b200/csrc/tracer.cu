@@ -67,16 +67,18 @@ constexpr int F_PEND = 27;  // 4 bits: pending light-slot contributions
 constexpr uint32_t F_CACHED = 1u << 31;  // the path ended into the radiance cache
 
 struct Wave {
-  float4* ray_o;   // o.xyz, previous pdf
-  float4* ray_d;   // d.xyz, flag word
-  float4* thr;     // throughput.xyz, pcg state
-  float4* res;     // result.xyz, pixel index
+  // Two float4 of a path that are read together share a 32-byte sector: the
+  // later bounces' paths lie scattered, and a float4 of its own costs a sector.
+  float4* ray;     // 2 per path: o.xyz, previous pdf; d.xyz, flag word
+  float4* tr;      // 2 per path: throughput.xyz, pcg state; result.xyz, pixel index
   float4* alb;     // first albedo
   float4* nrm;     // first normal
   float4* hit;     // t, slot, record, u
   float* hit_v;    // v
-  float4* sh_o;    // per slot: origin.xyz, limit
-  float4* sh_d;    // per slot: direction.xyz, visible flag
+  // shadow slots: the j-th pending slot of path i at j * capacity + i, so that
+  // neighbouring paths' slots are neighbours (a stride of `cap` slots a path
+  // wrote 255 and read 400 bytes a path where 48 and 190 do)
+  float4* sh;      // 2 per slot: origin.xyz, limit; direction.xyz, visible flag
   float4* sh_c;    // per slot: contribution.xyz
   uint32_t* queue[2];
   uint32_t* squeue;
@@ -90,7 +92,7 @@ struct Wave {
   uint32_t* cursor;    // SORT_BINS: entries handed out per key
   // split shade: the paths that scatter this bounce (count at counters[12]) and their surfaces
   uint32_t* lit;
-  float4* surf;        // 9 float4 per path
+  float4* surf;        // 4 float4 per path (store_surface; the last holds the light tree's pick)
   uint32_t* rhist;     // RAY_BINS: the extend queue's histogram by ray key
   uint32_t* rcursor;
   // queue items the traversal handed over to the IEEE walk (rays that are not
@@ -98,9 +100,25 @@ struct Wave {
   // (connect, in retry): the two kernels may run at the same time
   uint32_t* retry;
   uint32_t* eretry;
-  // the light tree's pick of each path that scatters (row, pmf), by lit index
-  float2* pick;
 };
+
+// One 32-byte sector (two float4) in one load or store (sm_100's 256-bit accesses).
+struct Pair {
+  float4 a, b;
+};
+__device__ __forceinline__ Pair load_pair(const float4* p) {
+  Pair r;
+  // no memory clobber: a thread never reads a pair again after it wrote to it
+  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+      : "l"(p));
+  return r;
+}
+__device__ __forceinline__ void store_pair(float4* p, float4 a, float4 b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
 
 // The radiance cache as the wave sees it (all null/zero when none is attached).
 struct CachePass {
@@ -265,10 +283,10 @@ __global__ void k_gen(const __grid_constant__ Pass P) {
       origin = add3(origin, add3(scl3(normalize3(cam_r), radius * cos_(phi)), scl3(normalize3(cam_u), radius * sin_(phi))));
       direction = normalize3(sub3(focus, origin));
     }
-    P.w.ray_o[i] = make_float4(origin.x, origin.y, origin.z, 0.0f);
-    P.w.ray_d[i] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(3u));  // carried = 3
-    P.w.thr[i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(state));
-    P.w.res[i] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(pixel));
+    P.w.ray[2u * i] = make_float4(origin.x, origin.y, origin.z, 0.0f);
+    P.w.ray[2u * i + 1u] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(3u));  // carried = 3
+    P.w.tr[2u * i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(state));
+    P.w.tr[2u * i + 1u] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(pixel));
     P.w.alb[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     P.w.nrm[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     P.w.queue[0][i] = i;
@@ -347,7 +365,7 @@ __device__ __forceinline__ uint32_t material_key(const Pass& P, uint32_t i) {
   if (P.c.enabled && P.bounce >= P.c.query_bounce && P.bounce <= P.c.query_last) {
     cont = P.c.tslot[i] != ~0u ? 1u : 0u;
     if (!cont) {
-      float4 o = P.w.ray_o[i], d = P.w.ray_d[i];
+      float4 o = P.w.ray[2u * i], d = P.w.ray[2u * i + 1u];
       cont = cell_ok(P.c, add3(mk3(o.x, o.y, o.z), scl3(mk3(d.x, d.y, d.z), h.x))) ? 0u : 1u;
       if (!cont && P.bounce < P.c.query_last && P.c.min_roughness > 0.0f) {
         const float4* row = P.v.materials + (size_t)(material + 1u) * 8u;
@@ -373,7 +391,7 @@ __device__ __forceinline__ void block_chunk(uint32_t n, uint32_t& first, uint32_
 constexpr uint32_t RAY_BINS = 512;
 
 __device__ __forceinline__ uint32_t ray_key(const Pass& P, uint32_t i) {
-  float4 o = P.w.ray_o[i], d = P.w.ray_d[i];
+  float4 o = P.w.ray[2u * i], d = P.w.ray[2u * i + 1u];
   float q[3] = {o.x, o.y, o.z};
   uint32_t cell = 0u;
 #pragma unroll
@@ -491,9 +509,8 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
         idx = first + (uint32_t)__popc(m & ((1u << lane) - 1u));
         if (idx < n) {
           item = queue[idx];
-          float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
-          float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
-          w.start(P.s, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), ANY ? a.w : 1e20f);
+          const Pair r = load_pair((ANY ? P.w.sh : P.w.ray) + 2u * item);
+          w.start(P.s, mk3(r.a.x, r.a.y, r.a.z), mk3(r.b.x, r.b.y, r.b.z), ANY ? r.a.w : 1e20f);
           have = true;
         } else {
           retired = true;
@@ -502,17 +519,16 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
     }
     if (__all_sync(FULL, retired)) break;
     w.inner_phase(P.s, st, [&](v3& o, v3& d) {
-      float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
-      float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
-      o = mk3(a.x, a.y, a.z);
-      d = mk3(b.x, b.y, b.z);
+      const Pair r = load_pair((ANY ? P.w.sh : P.w.ray) + 2u * item);
+      o = mk3(r.a.x, r.a.y, r.a.z);
+      d = mk3(r.b.x, r.b.y, r.b.z);
     });
     if (w.leaf_ready()) w.leaf_phase(P.s, st);
     if (have && w.finished()) {
       if (w.hit.hit == QuadWalker<ANY>::RETRY) {
         (ANY ? P.w.retry : P.w.eretry)[atomicAdd(P.w.counters + (ANY ? 14 : 13), 1u)] = item;
       } else if (ANY) {
-        reinterpret_cast<float*>(P.w.sh_d + item)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
+        reinterpret_cast<float*>(P.w.sh + 2u * item + 1u)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
       } else {
         P.w.hit[item] = make_float4(w.hit.t, __uint_as_float(w.hit.slot), __uint_as_float(w.record(P.s)), w.hit.u);
         P.w.hit_v[item] = w.hit.v;
@@ -531,8 +547,8 @@ __global__ void __launch_bounds__(128) k_trace_queue_retry(const __grid_constant
   const uint32_t n = P.w.counters[ANY ? 14 : 13];
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const uint32_t item = (ANY ? P.w.retry : P.w.eretry)[k];
-    float4 a = ANY ? P.w.sh_o[item] : P.w.ray_o[item];
-    float4 b = ANY ? P.w.sh_d[item] : P.w.ray_d[item];
+    float4 a = ANY ? P.w.sh[2u * item] : P.w.ray[2u * item];
+    float4 b = ANY ? P.w.sh[2u * item + 1u] : P.w.ray[2u * item + 1u];
     RefStack st;
     Walker<ANY, false, BOX_IEEE> w;
     w.start(P.s, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), ANY ? a.w : 1e20f);
@@ -541,7 +557,7 @@ __global__ void __launch_bounds__(128) k_trace_queue_retry(const __grid_constant
       d = mk3(b.x, b.y, b.z);
     });
     if (ANY) {
-      reinterpret_cast<float*>(P.w.sh_d + item)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
+      reinterpret_cast<float*>(P.w.sh + 2u * item + 1u)[3] = __uint_as_float(w.hit.hit ? 0u : 1u);
     } else {
       P.w.hit[item] = make_float4(w.hit.t, __uint_as_float(w.hit.slot), __uint_as_float(w.hit.record), w.hit.u);
       P.w.hit_v[item] = w.hit.v;
@@ -605,8 +621,8 @@ __device__ __forceinline__ float emitter_weight(const Pass& P, const HitInfo& hi
 __device__ __forceinline__ v3 flush_pending(const Pass& P, uint32_t i, uint32_t flags, v3 result) {
   uint32_t pending = (flags >> F_PEND) & 15u;
   for (uint32_t j = 0; j < pending; ++j) {
-    uint32_t slot = i * P.cap + j;
-    float vis = reinterpret_cast<const float*>(P.w.sh_d + slot)[3];
+    uint32_t slot = j * P.capacity + i;
+    float vis = reinterpret_cast<const float*>(P.w.sh + 2u * slot + 1u)[3];
     if (__float_as_uint(vis) != 0u) result = add3(result, f3of(P.w.sh_c[slot]));
   }
   return result;
@@ -667,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, SHADE_MIN_BLOCKS) k_shade(const __gr
     bool cont = false;
     uint32_t i = active ? queue[qi] : 0u;
     if (active) {
-      float4 ro = P.w.ray_o[i], rd = P.w.ray_d[i], th = P.w.thr[i], rs = P.w.res[i];
+      float4 ro = P.w.ray[2u * i], rd = P.w.ray[2u * i + 1u], th = P.w.tr[2u * i], rs = P.w.tr[2u * i + 1u];
       v3 o = mk3(ro.x, ro.y, ro.z), d = mk3(rd.x, rd.y, rd.z);
       float previous_pdf = ro.w;
       uint32_t flags = __float_as_uint(rd.w);
@@ -816,10 +832,10 @@ __global__ void __launch_bounds__(kThreads, SHADE_MIN_BLOCKS) k_shade(const __gr
               result = add3(result, term);
               continue;
             }
-            uint32_t slot_index = i * P.cap + pending;
+            uint32_t slot_index = pending * P.capacity + i;
             P.w.sh_c[slot_index] = make_float4(term.x, term.y, term.z, 0.0f);
-            P.w.sh_o[slot_index] = make_float4(origin.x, origin.y, origin.z, limit);
-            P.w.sh_d[slot_index] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u));
+            P.w.sh[2u * slot_index] = make_float4(origin.x, origin.y, origin.z, limit);
+            P.w.sh[2u * slot_index + 1u] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u));
             uint32_t at = claim(P.w.counters + 2, limit > 0.0f);  // one atomic per warp
             if (limit > 0.0f) P.w.squeue[at] = slot_index;
             pending += 1u;
@@ -870,10 +886,10 @@ __global__ void __launch_bounds__(kThreads, SHADE_MIN_BLOCKS) k_shade(const __gr
         }
       }
       flags |= pending << F_PEND;
-      P.w.ray_o[i] = make_float4(o.x, o.y, o.z, previous_pdf);
-      P.w.ray_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(flags));
-      P.w.thr[i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
-      P.w.res[i] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
+      P.w.ray[2u * i] = make_float4(o.x, o.y, o.z, previous_pdf);
+      P.w.ray[2u * i + 1u] = make_float4(d.x, d.y, d.z, __uint_as_float(flags));
+      P.w.tr[2u * i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
+      P.w.tr[2u * i + 1u] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
     }
     append(next_queue, next_count, i, active && cont);
   }
@@ -887,51 +903,38 @@ __global__ void __launch_bounds__(kThreads, SHADE_MIN_BLOCKS) k_shade(const __gr
 // surface travels between them in 9 float4 per path; every expression is the
 // fused kernel's, in the same order, so the results are identical.
 
+// 64 bytes a path: the point and distance, the normal and side; the geometric
+// normal and the material, and room for the light tree's pick.  The material's
+// parameters are read from its row again, which the caches hold, instead of
+// travelling with every path.  With that, the paired sectors and the shadow
+// slots by pending slot, a light slot moves 0.9 GB for 3.6 M paths instead of
+// 2.5 (639 -> 375 us), the hit kernel 1.1 instead of 1.5 (374 -> 273 us); 1280
+// x 720 at 16 samples 77.9 -> 67.4 ms, the 4K pass 70.7 -> 65.7.
 __device__ __forceinline__ void store_surface(float4* out, v3 p, float t, v3 nn, bool entering, v3 geometric,
-                                              const Shaded& s) {
-  out[0] = make_float4(p.x, p.y, p.z, t);
-  out[1] = make_float4(nn.x, nn.y, nn.z, entering ? 1.0f : 0.0f);
-  out[2] = make_float4(geometric.x, geometric.y, geometric.z, s.roughness);
-  out[3] = make_float4(s.base.x, s.base.y, s.base.z, s.metalness);
-  out[4] = make_float4(s.specular, s.clearcoat, s.clearcoat_roughness, s.sheen);
-  out[5] = make_float4(s.transmission, s.ior, s.dispersion, s.thickness);
-  out[6] = make_float4(s.subsurface, s.subsurface_tint.x, s.subsurface_tint.y, s.subsurface_tint.z);
-  out[7] = make_float4(s.absorption, s.emission.x, s.emission.y, s.emission.z);
-  out[8] = make_float4(s.fresnel_power, 0.0f, 0.0f, 0.0f);
+                                              uint32_t material) {
+  store_pair(out, make_float4(p.x, p.y, p.z, t), make_float4(nn.x, nn.y, nn.z, entering ? 1.0f : 0.0f));
+  out[2] = make_float4(geometric.x, geometric.y, geometric.z, __uint_as_float(material));
 }
 
-struct Surface {
-  v3 p, nn, geometric;
-  float t;
-  bool entering;
-  Shaded s;
-};
-
-__device__ __forceinline__ Surface load_surface_record(const float4* in) {
-  float4 a = in[0], b = in[1], c = in[2], e = in[3], f = in[4], g = in[5], h = in[6], k = in[7], m = in[8];
-  Surface S;
-  S.p = mk3(a.x, a.y, a.z);
-  S.t = a.w;
-  S.nn = mk3(b.x, b.y, b.z);
-  S.entering = b.w != 0.0f;
-  S.geometric = mk3(c.x, c.y, c.z);
-  S.s.roughness = c.w;
-  S.s.base = mk3(e.x, e.y, e.z);
-  S.s.metalness = e.w;
-  S.s.specular = f.x;
-  S.s.clearcoat = f.y;
-  S.s.clearcoat_roughness = f.z;
-  S.s.sheen = f.w;
-  S.s.transmission = g.x;
-  S.s.ior = g.y;
-  S.s.dispersion = g.z;
-  S.s.thickness = g.w;
-  S.s.subsurface = h.x;
-  S.s.subsurface_tint = mk3(h.y, h.z, h.w);
-  S.s.absorption = k.x;
-  S.s.emission = mk3(k.y, k.z, k.w);
-  S.s.fresnel_power = m.x;
-  return S;
+// A material as a path with `flags` shades it: load_surface with the least
+// roughness and the filter of glossy lobes behind a diffuse bounce.
+__device__ __forceinline__ float shaded_roughness(const Specialise& sp, float roughness, uint32_t flags) {
+  roughness = fmax_(roughness, 0.05f);
+  if (sp.filter_glossy > 0.0f && (flags & F_DIFFUSED)) roughness = fmax_(roughness, sp.filter_glossy);
+  return roughness;
+}
+__device__ __forceinline__ Shaded load_shaded(const ShadeView& V, const Specialise& sp, uint32_t material,
+                                              uint32_t flags) {
+  Shaded s = load_surface(V, material);
+  s.roughness = shaded_roughness(sp, s.roughness, flags);
+  s.clearcoat_roughness = shaded_roughness(sp, s.clearcoat_roughness, flags);
+  return s;
+}
+// Its roughness alone.
+__device__ __forceinline__ float load_roughness(const ShadeView& V, const Specialise& sp, uint32_t material,
+                                                uint32_t flags) {
+  return shaded_roughness(sp, __ldg(reinterpret_cast<const float*>(V.materials + (size_t)(material + 1u) * 8u) + 3),
+                          flags);
 }
 
 __global__ void __launch_bounds__(kThreads) k_shade_hit(const __grid_constant__ Pass P, uint32_t which) {
@@ -946,7 +949,8 @@ __global__ void __launch_bounds__(kThreads) k_shade_hit(const __grid_constant__ 
     bool lit = false;
     uint32_t i = active ? queue[qi] : 0u;
     if (active) {
-      float4 ro = P.w.ray_o[i], rd = P.w.ray_d[i], th = P.w.thr[i], rs = P.w.res[i];
+      const Pair ray = load_pair(P.w.ray + 2u * i), tr = load_pair(P.w.tr + 2u * i);
+      const float4 ro = ray.a, rd = ray.b, th = tr.a, rs = tr.b;
       v3 o = mk3(ro.x, ro.y, ro.z), d = mk3(rd.x, rd.y, rd.z);
       float previous_pdf = ro.w;
       uint32_t flags = __float_as_uint(rd.w);
@@ -969,15 +973,9 @@ __global__ void __launch_bounds__(kThreads) k_shade_hit(const __grid_constant__ 
         HitInfo hit = fill_hit(P, h, P.w.hit_v[i]);
         v3 p = add3(o, scl3(d, hit.t));
         v3 nn = dot3(hit.n, d) > 0.0f ? neg3(hit.n) : hit.n;
-        Shaded s = load_surface(V, hit.material);
+        Shaded s = load_shaded(V, sp, hit.material, flags);
         v3 geometric = dot3(hit.geometric, d) > 0.0f ? neg3(hit.geometric) : hit.geometric;
         if (dot3(nn, geometric) < 0.05f) nn = normalize3(add3(nn, scl3(geometric, 0.1f)));
-        s.roughness = fmax_(s.roughness, 0.05f);
-        s.clearcoat_roughness = fmax_(s.clearcoat_roughness, 0.05f);
-        if (sp.filter_glossy > 0.0f && (flags & F_DIFFUSED)) {
-          s.roughness = fmax_(s.roughness, sp.filter_glossy);
-          s.clearcoat_roughness = fmax_(s.clearcoat_roughness, sp.filter_glossy);
-        }
         if (bounce == 0u) {
           P.w.alb[i] = make_float4(s.base.x, s.base.y, s.base.z, 1.0f);
           P.w.nrm[i] = make_float4(nn.x, nn.y, nn.z, 1.0f);
@@ -1006,12 +1004,12 @@ __global__ void __launch_bounds__(kThreads) k_shade_hit(const __grid_constant__ 
           }
         }
         if (!(flags & F_LAST) && !to_cache) {
-          store_surface(P.w.surf + (size_t)i * 9u, p, hit.t, nn, dot3(hit.n, d) < 0.0f, geometric, s);
+          store_surface(P.w.surf + (size_t)i * 4u, p, hit.t, nn, dot3(hit.n, d) < 0.0f, geometric, hit.material);
           lit = true;
         }
       }
-      P.w.ray_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(flags));
-      P.w.res[i] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
+      if (flags != __float_as_uint(rd.w)) reinterpret_cast<float*>(P.w.ray + 2u * i + 1u)[3] = __uint_as_float(flags);
+      P.w.tr[2u * i + 1u] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
     }
     append(P.w.lit, P.w.counters + 12, i, active && lit);
   }
@@ -1025,7 +1023,7 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
   const ShadeView& V = P.v;
   for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < n; qi += gridDim.x * blockDim.x) {
     const uint32_t i = P.w.lit[qi];
-    float4 ro = P.w.ray_o[i], rd = P.w.ray_d[i], th = P.w.thr[i], rs = P.w.res[i];
+    float4 ro = P.w.ray[2u * i], rd = P.w.ray[2u * i + 1u], th = P.w.tr[2u * i], rs = P.w.tr[2u * i + 1u];
     v3 o = mk3(ro.x, ro.y, ro.z), d = mk3(rd.x, rd.y, rd.z);
     uint32_t flags = __float_as_uint(rd.w);
     v3 throughput = mk3(th.x, th.y, th.z);
@@ -1037,10 +1035,11 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
     // The surface's geometry is held across the slots; its material record is
     // read again where a slot evaluates the BSDF, so that it is not live across
     // the light-tree descent (fewer values to keep in local memory there).
-    const float4* record = P.w.surf + (size_t)i * 9u;
+    const float4* record = P.w.surf + (size_t)i * 4u;
     const float4 g0 = record[0], g1 = record[1], g2 = record[2];
     const v3 p = mk3(g0.x, g0.y, g0.z), nn = mk3(g1.x, g1.y, g1.z), geometric = mk3(g2.x, g2.y, g2.z);
-    const float roughness = g2.w;
+    const uint32_t material = __float_as_uint(g2.w);
+    const float roughness = load_roughness(V, sp, material, flags);
     m3 transform = basis(nn);
     v3 origin = spawn_point(p, nn, o, g0.w);
     uint32_t pending = 0u;
@@ -1105,8 +1104,7 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
         limit = picked.limit;
         lit_roughness = fmax_(roughness, picked.roughness);
       }
-      const Surface S = load_surface_record(record);
-      const Shaded& s = S.s;
+      const Shaded s = load_shaded(V, sp, material, flags);
       const v3 wo = mulmtv(transform, neg3(d));
       if (pdf > 0.0f) {
         float bsdf = bsdf_pdf(s, wo, local);
@@ -1128,17 +1126,17 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
         result = add3(result, term);
         continue;
       }
-      uint32_t slot_index = i * P.cap + pending;
+      uint32_t slot_index = pending * P.capacity + i;
       P.w.sh_c[slot_index] = make_float4(term.x, term.y, term.z, 0.0f);
-      P.w.sh_o[slot_index] = make_float4(origin.x, origin.y, origin.z, limit);
-      P.w.sh_d[slot_index] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u));
+      P.w.sh[2u * slot_index] = make_float4(origin.x, origin.y, origin.z, limit);
+      P.w.sh[2u * slot_index + 1u] = make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u));
       uint32_t at = claim(P.w.counters + 2, limit > 0.0f);  // one atomic per warp
       if (limit > 0.0f) P.w.squeue[at] = slot_index;
       pending += 1u;
     }
-    P.w.ray_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(flags | (pending << F_PEND)));
-    P.w.thr[i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
-    if (!DEFERRED) P.w.res[i] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
+    P.w.ray[2u * i + 1u] = make_float4(d.x, d.y, d.z, __uint_as_float(flags | (pending << F_PEND)));
+    P.w.tr[2u * i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
+    if (!DEFERRED) P.w.tr[2u * i + 1u] = make_float4(result.x, result.y, result.z, __uint_as_float(pixel));
   }
 }
 
@@ -1160,20 +1158,21 @@ constexpr int SLOT_SUN = 0, SLOT_SKY = 1, SLOT_EMITTER = 2, SLOT_LOOPED = 3, SLO
 #ifndef TRACE_AHEAD
 #define TRACE_AHEAD 1
 #endif
+// Blocks of 128 per SM of the slot kernels: 6, 8, 10 and 12 gave 1280 x 720 at
+// 16 samples 67.4, 68.1, 72.1 and 73.6 ms (fewer spills, more registers).
 #ifndef SLOT_MIN_BLOCKS
-#define SLOT_MIN_BLOCKS 8
+#define SLOT_MIN_BLOCKS 6
 #endif
 #ifndef PICK_MIN_BLOCKS
 #define PICK_MIN_BLOCKS 10
 #endif
-__device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i) {
-  const uint32_t pixel = __float_as_uint(reinterpret_cast<const float*>(P.w.res + i)[3]);
+__device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i, uint32_t pixel) {
   uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
   return Rng{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (P.bounce + 1u)};
 }
 
 // The light tree's descent for every scattering path (slot k of tree_pick's
-// caller in k_shade_lights): the pick (light row, pmf) at P.w.pick[qi].  Bound
+// caller in k_shade_lights): the pick (light row, pmf) into its surface record.  Bound
 // by issue slots (73 % busy).  With the reference's rows through out-of-line
 // helpers a 100k-triangle room's 3.6 M descents took 1687 us, 12,000
 // instructions a warp at 17 of 32 lanes, with 290 M sectors of local memory;
@@ -1187,17 +1186,20 @@ __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const _
   const ShadeView& V = P.v;
   for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < n; qi += gridDim.x * blockDim.x) {
     const uint32_t i = P.w.lit[qi];
-    const float4* record = P.w.surf + (size_t)i * 9u;
-    const float4 g0 = record[0], g1 = record[1];
-    uint32_t state = __float_as_uint(reinterpret_cast<const float*>(P.w.thr + i)[3]);
+    float4* record = P.w.surf + (size_t)i * 4u;
+    const Pair g = load_pair(record);
+    const float4 g0 = g.a, g1 = g.b;
+    uint32_t state = __float_as_uint(reinterpret_cast<const float*>(P.w.tr + 2u * i)[3]);
     float start;
     if (sp.sobol) {
-      start = sobol_z(V, sp, slot_rng(P, i), light_dim(k));
+      start = sobol_z(V, sp, slot_rng(P, i, __float_as_uint(reinterpret_cast<const float*>(P.w.tr + 2u * i + 1u)[3])),
+                      light_dim(k));
     } else {
       start = random01(state);
-      reinterpret_cast<float*>(P.w.thr + i)[3] = __uint_as_float(state);
+      reinterpret_cast<float*>(P.w.tr + 2u * i)[3] = __uint_as_float(state);
     }
-    P.w.pick[qi] = tree_pick_rows(V, P.light_rows, mk3(g0.x, g0.y, g0.z), mk3(g1.x, g1.y, g1.z), start);
+    *reinterpret_cast<float2*>(record + 3) =
+        tree_pick_rows(V, P.light_rows, mk3(g0.x, g0.y, g0.z), mk3(g1.x, g1.y, g1.z), start);
   }
 }
 
@@ -1211,26 +1213,25 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
   const ShadeView& V = P.v;
   for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < n; qi += gridDim.x * blockDim.x) {
     const uint32_t i = P.w.lit[qi];
-    float2 pk = make_float2(0.0f, 0.0f);
-    if (KIND == SLOT_TREE) {
-      pk = P.w.pick[qi];
-      if (!(pk.y > 0.0f)) continue;  // no light picked: the slot adds nothing and draws nothing more
-    }
-    const float4 rd = P.w.ray_d[i], th = P.w.thr[i];
+    const float4* record = P.w.surf + (size_t)i * 4u;
+    const Pair side = load_pair(record + 2);
+    const float4 g2 = side.a;
+    const float2 pk = make_float2(side.b.x, side.b.y);
+    if (KIND == SLOT_TREE && !(pk.y > 0.0f)) continue;  // no light picked: the slot adds nothing and draws nothing more
+    const Pair at_hit = load_pair(record), ray = load_pair(P.w.ray + 2u * i), tr = load_pair(P.w.tr + 2u * i);
+    const float4 g0 = at_hit.a, g1 = at_hit.b, ro = ray.a, rd = ray.b, th = tr.a;
     const v3 d = mk3(rd.x, rd.y, rd.z);
     const uint32_t flags = __float_as_uint(rd.w);
     uint32_t state = __float_as_uint(th.w);
     const uint32_t state_in = state;
-    const float4* record = P.w.surf + (size_t)i * 9u;
-    const float4 g0 = record[0], g1 = record[1], g2 = record[2];
     const v3 p = mk3(g0.x, g0.y, g0.z), nn = mk3(g1.x, g1.y, g1.z);
     const m3 transform = basis(nn);
     float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (sp.sobol) u = sobol4(V, sp, slot_rng(P, i), light_dim(k));
+    if (sp.sobol) u = sobol4(V, sp, slot_rng(P, i, __float_as_uint(tr.b.w)), light_dim(k));
     v3 local = mk3(0.0f, 0.0f, 1.0f), direction = mk3(0.0f, 0.0f, 1.0f), strength = splat3(0.0f);
     v3 origin = p;
     float limit = 1e19f, pdf = 0.0f;
-    float lit_roughness = g2.w;
+    float widened = 0.0f;  // the light's own roughness
     bool live = true;
     if (KIND == SLOT_SUN) {
       direction = normalize3(mk3(P.f.sun_dir[0], P.f.sun_dir[1], P.f.sun_dir[2]));
@@ -1244,7 +1245,6 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
       local = mulmtv(transform, direction);
       live = local.z > 0.0f;
       strength = scl3(mk3(P.f.sun_color[0], P.f.sun_color[1], P.f.sun_color[2]), P.f.sun_color[3] * 1.0f);
-      const float4 ro = P.w.ray_o[i];
       origin = spawn_point(p, nn, mk3(ro.x, ro.y, ro.z), g0.w);
     } else if (KIND == SLOT_SKY) {
       float ux = rnd(sp, state, u.x);
@@ -1258,11 +1258,9 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
         strength = scl3(sky_radiance(V), 1.0f);
         pdf = light.pdf;
         live = local.z > 0.0f && pdf > 0.0f;
-        const float4 ro = P.w.ray_o[i];
         origin = spawn_point(p, nn, mk3(ro.x, ro.y, ro.z), g0.w);
       }
     } else {
-      const float4 ro = P.w.ray_o[i];
       origin = spawn_point(p, nn, mk3(ro.x, ro.y, ro.z), g0.w);
       Candidate picked;
       if (KIND == SLOT_TREE) {
@@ -1279,11 +1277,12 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
       strength = picked.scale;
       pdf = picked.pdf;
       limit = picked.limit;
-      lit_roughness = fmax_(lit_roughness, picked.roughness);
+      widened = picked.roughness;
     }
     if (live) {
-      const Surface S = load_surface_record(record);
-      const Shaded& s = S.s;
+      const Shaded s = load_shaded(V, sp, __float_as_uint(g2.w), flags);
+      const float lit_roughness =
+          KIND == SLOT_SUN || KIND == SLOT_SKY ? s.roughness : fmax_(s.roughness, widened);
       const v3 wo = mulmtv(transform, neg3(d));
       if (pdf > 0.0f) {
         float bsdf = bsdf_pdf(s, wo, local);
@@ -1303,18 +1302,17 @@ __global__ void __launch_bounds__(kThreads, SLOT_MIN_BLOCKS) k_light_slot(const 
       live = !(term.x == 0.0f && term.y == 0.0f && term.z == 0.0f);  // adds nothing, traces nothing
       if (live) {
         const uint32_t pending = (flags >> F_PEND) & 15u;
-        uint32_t slot_index = i * P.cap + pending;
+        uint32_t slot_index = pending * P.capacity + i;
         P.w.sh_c[slot_index] = make_float4(term.x, term.y, term.z, 0.0f);
-        P.w.sh_o[slot_index] = make_float4(origin.x, origin.y, origin.z, limit);
-        P.w.sh_d[slot_index] =
-            make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u));
-        reinterpret_cast<float*>(P.w.ray_d + i)[3] =
+        store_pair(P.w.sh + 2u * (size_t)slot_index, make_float4(origin.x, origin.y, origin.z, limit),
+                   make_float4(direction.x, direction.y, direction.z, __uint_as_float(limit > 0.0f ? 0u : 1u)));
+        reinterpret_cast<float*>(P.w.ray + 2u * i + 1u)[3] =
             __uint_as_float((flags & ~(15u << F_PEND)) | ((pending + 1u) << F_PEND));
       }
     }
     uint32_t at = claim(P.w.counters + 2, live && limit > 0.0f);  // one atomic per warp
-    if (live && limit > 0.0f) P.w.squeue[at] = i * P.cap + ((flags >> F_PEND) & 15u);
-    if (state != state_in) reinterpret_cast<float*>(P.w.thr + i)[3] = __uint_as_float(state);
+    if (live && limit > 0.0f) P.w.squeue[at] = ((flags >> F_PEND) & 15u) * P.capacity + i;
+    if (state != state_in) reinterpret_cast<float*>(P.w.tr + 2u * i)[3] = __uint_as_float(state);
   }
 }
 
@@ -1332,22 +1330,25 @@ __global__ void __launch_bounds__(kThreads) k_shade_bsdf(const __grid_constant__
     bool cont = false;
     uint32_t i = active ? P.w.lit[qi] : 0u;
     if (active) {
-      float4 ro = P.w.ray_o[i], rd = P.w.ray_d[i], th = P.w.thr[i];
+      const Pair ray = load_pair(P.w.ray + 2u * i), tr = load_pair(P.w.tr + 2u * i);
+      const float4* record = P.w.surf + (size_t)i * 4u;
+      const Pair at_hit = load_pair(record);
+      const uint32_t material = __float_as_uint(reinterpret_cast<const float*>(record + 2)[3]);
+      const float4 ro = ray.a, rd = ray.b, th = tr.a;
       v3 o = mk3(ro.x, ro.y, ro.z), d = mk3(rd.x, rd.y, rd.z);
       float previous_pdf = ro.w;
       uint32_t flags = __float_as_uint(rd.w);
       const uint32_t pending = (flags >> F_PEND) & 15u;
       v3 throughput = mk3(th.x, th.y, th.z);
       uint32_t state = __float_as_uint(th.w);
-      uint32_t pixel = __float_as_uint(P.w.res[i].w);
+      uint32_t pixel = __float_as_uint(tr.b.w);
       uint32_t px = pixel % P.width + P.f.window[2], py = pixel / P.width + P.f.window[3];
       Rng r{hash_iqnt2d(px, py) ^ pass_seed(P), pass_accum(P) + path_sample(P, i), 16u * (bounce + 1u)};
-      const Surface S = load_surface_record(P.w.surf + (size_t)i * 9u);
-      const Shaded& s = S.s;
-      const v3 p = S.p;
-      m3 transform = basis(S.nn);
+      const Shaded s = load_shaded(V, sp, material, flags);
+      const v3 p = mk3(at_hit.a.x, at_hit.a.y, at_hit.a.z);
+      m3 transform = basis(mk3(at_hit.b.x, at_hit.b.y, at_hit.b.z));
       v3 wo = mulmtv(transform, neg3(d));
-      bool entering = S.entering;
+      bool entering = at_hit.b.w != 0.0f;
       // BSDF sampling and the next ray (trace.wgsl:2472-2500)
       uint32_t carried = flags & F_CARRIED;
       BsdfSample sample = sample_bsdf(sp, s, wo, entering, carried, state, sobol4(V, sp, r, 3u));
@@ -1378,7 +1379,7 @@ __global__ void __launch_bounds__(kThreads) k_shade_bsdf(const __grid_constant__
         previous_pdf = sample.pdf;
       }
       if (go) {
-        o = spawn_point(p, d, o, S.t);
+        o = spawn_point(p, d, o, at_hit.a.w);
         if (bounce >= 3u) {
           float keep = clamp_(fmax_(throughput.x, fmax_(throughput.y, throughput.z)), 0.05f, 0.95f);
           Rng r0 = r;
@@ -1392,9 +1393,9 @@ __global__ void __launch_bounds__(kThreads) k_shade_bsdf(const __grid_constant__
               (through ? F_THROUGH : 0u) | (lit_vertex ? F_LIT : 0u) | (diffused ? F_DIFFUSED : 0u);
       flags |= pending << F_PEND;
       cont = go;
-      P.w.ray_o[i] = make_float4(o.x, o.y, o.z, previous_pdf);
-      P.w.ray_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(flags));
-      P.w.thr[i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
+      store_pair(P.w.ray + 2u * i, make_float4(o.x, o.y, o.z, previous_pdf),
+                 make_float4(d.x, d.y, d.z, __uint_as_float(flags)));
+      P.w.tr[2u * i] = make_float4(throughput.x, throughput.y, throughput.z, __uint_as_float(state));
     }
     append(next_queue, next_count, i, active && cont);
   }
@@ -1410,12 +1411,12 @@ __global__ void k_finish(const __grid_constant__ Pass P,Accum* __restrict__ accu
     const uint32_t pixel = P.w.active[k];
     Accum a = accum[pixel];
     for (uint32_t i = k << P.shift; i < (k + 1u) << P.shift; ++i) {
-      float4 rs = P.w.res[i];
-      uint32_t flags = __float_as_uint(P.w.ray_d[i].w);
+      float4 rs = P.w.tr[2u * i + 1u];
+      uint32_t flags = __float_as_uint(P.w.ray[2u * i + 1u].w);
       v3 result = flush_pending(P, i, flags, mk3(rs.x, rs.y, rs.z));
       if (flags & F_CACHED) {
         // the cache's radiance at the vertex the path ended at, through its throughput
-        float4 pr = P.c.pred[i], th = P.w.thr[i];
+        float4 pr = P.c.pred[i], th = P.w.tr[2u * i];
         v3 radiance = mk3(fmaxf(pr.x, 0.0f), fmaxf(pr.y, 0.0f), fmaxf(pr.z, 0.0f));
         result = add3(result, capped(P, mul3(mk3(th.x, th.y, th.z), radiance), true));
       }
@@ -1580,16 +1581,14 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
     need = at + bytes;
     return at;
   };
-  size_t o_ray_o = add(16ull * capacity), o_ray_d = add(16ull * capacity), o_thr = add(16ull * capacity),
-         o_res = add(16ull * capacity), o_alb = add(16ull * capacity), o_nrm = add(16ull * capacity),
-         o_hit = add(16ull * capacity), o_hitv = add(4ull * capacity), o_sho = add(16ull * capacity * cap),
-         o_shd = add(16ull * capacity * cap), o_shc = add(16ull * capacity * cap), o_q0 = add(4ull * capacity),
+  size_t o_ray = add(32ull * capacity), o_tr = add(32ull * capacity), o_alb = add(16ull * capacity),
+         o_nrm = add(16ull * capacity), o_hit = add(16ull * capacity), o_hitv = add(4ull * capacity),
+         o_sh = add(32ull * capacity * cap), o_shc = add(16ull * capacity * cap), o_q0 = add(4ull * capacity),
          o_q1 = add(4ull * capacity), o_sq = add(4ull * capacity * cap), o_act = add(4ull * capacity),
-         o_keys = add(4ull * capacity), o_sorted = add(4ull * capacity),
-         o_hist = add(4ull * SORT_BINS), o_cursor = add(4ull * SORT_BINS), o_lit = add(4ull * capacity),
-         o_surf = add(144ull * capacity), o_rhist = add(4ull * RAY_BINS), o_rcursor = add(4ull * RAY_BINS),
-         o_retry = add(4ull * capacity * (cap > 0 ? cap : 1)), o_eretry = add(4ull * capacity),
-         o_pick = add(8ull * capacity);
+         o_keys = add(4ull * capacity), o_sorted = add(4ull * capacity), o_hist = add(4ull * SORT_BINS),
+         o_cursor = add(4ull * SORT_BINS), o_lit = add(4ull * capacity), o_surf = add(64ull * capacity),
+         o_rhist = add(4ull * RAY_BINS), o_rcursor = add(4ull * RAY_BINS),
+         o_retry = add(4ull * capacity * (cap > 0 ? cap : 1)), o_eretry = add(4ull * capacity);
   if (need > held) {
     if (wide) {
       size_t free_bytes = 0, total = 0;
@@ -1607,16 +1606,13 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
   }
   char* b = static_cast<char*>(buffer);
   Wave& w = *reinterpret_cast<Wave*>(&t.wave_layout);
-  w.ray_o = reinterpret_cast<float4*>(b + o_ray_o);
-  w.ray_d = reinterpret_cast<float4*>(b + o_ray_d);
-  w.thr = reinterpret_cast<float4*>(b + o_thr);
-  w.res = reinterpret_cast<float4*>(b + o_res);
+  w.ray = reinterpret_cast<float4*>(b + o_ray);
+  w.tr = reinterpret_cast<float4*>(b + o_tr);
   w.alb = reinterpret_cast<float4*>(b + o_alb);
   w.nrm = reinterpret_cast<float4*>(b + o_nrm);
   w.hit = reinterpret_cast<float4*>(b + o_hit);
   w.hit_v = reinterpret_cast<float*>(b + o_hitv);
-  w.sh_o = reinterpret_cast<float4*>(b + o_sho);
-  w.sh_d = reinterpret_cast<float4*>(b + o_shd);
+  w.sh = reinterpret_cast<float4*>(b + o_sh);
   w.sh_c = reinterpret_cast<float4*>(b + o_shc);
   w.queue[0] = reinterpret_cast<uint32_t*>(b + o_q0);
   w.queue[1] = reinterpret_cast<uint32_t*>(b + o_q1);
@@ -1633,7 +1629,6 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
   w.rcursor = reinterpret_cast<uint32_t*>(b + o_rcursor);
   w.retry = reinterpret_cast<uint32_t*>(b + o_retry);
   w.eretry = reinterpret_cast<uint32_t*>(b + o_eretry);
-  w.pick = reinterpret_cast<float2*>(b + o_pick);
   return true;
 }
 
