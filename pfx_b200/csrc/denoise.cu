@@ -144,10 +144,12 @@ uint32_t pad16(uint32_t c) { return (c + 15u) / 16u * 16u; }
 
 // The weights of one layer as conv kernels stage them: for each chunk of 16
 // padded input channels (the first source's padded channels, then the skip
-// source's), 9 taps x 2 groups of 8 channels x n output rows x 8 halves,
-//   index = (((chunk * 9 + tap) * 2 + group) * n + o) * 8 + j,
-// the K-major canonical layout of the B operand of one tap (rows = output
-// channels, 16-byte rows of 8 input channels).  Padding is zero.
+// source's), 3 columns kx of taps x 2 groups of 8 channels x 3 rows of taps from
+// ky = 2 to ky = 0 x n output channels x 8 halves,
+//   index = ((((chunk * 3 + kx) * 2 + group) * 3 + (2 - ky)) * n + o) * 8 + j,
+// the K-major canonical layout of a B operand whose rows are the output
+// channels of up to three taps (rows of 8 input channels, 16 bytes).  Padding
+// is zero.
 std::vector<uint16_t> conv_chunks(const DenoiseLayer& L, const Tensor& w) {
   const uint32_t chunks = (L.c0 + L.c1) / 16u, inputs = L.in0 + L.in1;
   std::vector<uint16_t> out((size_t)chunks * 9u * 2u * L.n * 8u, 0u);
@@ -164,7 +166,9 @@ std::vector<uint16_t> conv_chunks(const DenoiseLayer& L, const Tensor& w) {
               ch = L.in0 + (pc - L.c0);
             }
             if (ch < 0) continue;
-            out[((((size_t)k * 9u + t) * 2u + g) * L.n + o) * 8u + j] = w.half[((size_t)o * inputs + ch) * 9u + t];
+            const uint32_t ky = t / 3u, kx = t % 3u;
+            out[(((((size_t)k * 3u + kx) * 2u + g) * 3u + (2u - ky)) * L.n + o) * 8u + j] =
+                w.half[((size_t)o * inputs + ch) * 9u + t];
           }
   return out;
 }
@@ -310,8 +314,8 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, 
 #pragma unroll 1
     for (uint32_t j = 0; j < a.n; j += 16u) {
       float v0[16], v1[16];
-      umma::ld16(umma::taddr(tmem, warp * 32u, r0 * S::N_MAX + j), v0);
-      umma::ld16(umma::taddr(tmem, warp * 32u, (r0 + 1u) * S::N_MAX + j), v1);
+      umma::ld16(umma::taddr(tmem, warp * 32u, r0 * a.n + j), v0);
+      umma::ld16(umma::taddr(tmem, warp * 32u, (r0 + 1u) * a.n + j), v1);
       float b[16];
 #pragma unroll
       for (int c = 0; c < 16; ++c) b[c] = __ldg(a.bias + j + c);
@@ -367,7 +371,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, 
 // the CTA drains what it issued and reports it in a.error.
 template <class S>
 __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_constant__ ConvArgs a) {
-  constexpr uint32_t STAGE = S::STAGE, A_BYTES = S::A_BYTES, CTRL = S::CTRL, N_MAX = S::N_MAX, ROWS = S::ROWS;
+  constexpr uint32_t STAGE = S::STAGE, A_BYTES = S::A_BYTES, CTRL = S::CTRL, ROWS = S::ROWS;
   constexpr uint32_t NS = S::STAGES, TMEM_COLS = S::TMEM_COLS;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -427,17 +431,16 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
       // at compile time, so the lane issues ROWS x 18 MMAs back to back.
       const uint64_t hi_desc = umma::desc(base + s * STAGE, A_PLANE, 128u);
       const uint64_t lo_desc = umma::desc(base + s * STAGE + A_BYTES, A_PLANE, 128u);
-      const uint64_t w_desc = umma::desc(base + s * STAGE + 2u * A_BYTES, a.n * 16u, 128u);
-      const uint32_t w_step = (2u * a.n * 16u) >> 4;
+      const uint64_t w_desc = umma::desc(base + s * STAGE + 2u * A_BYTES, 3u * a.n * 16u, 128u);
       const uint32_t first = k == 0 ? 0u : 1u;
 #pragma unroll
       for (uint32_t r = 0; r < ROWS; ++r) {
 #pragma unroll
         for (uint32_t tap = 0; tap < 9; ++tap) {
           const uint32_t off = ((r + tap / 3u) * 2u * A_PLANE + (tap % 3u) * 16u) / 16u;
-          const uint64_t bd = w_desc + tap * w_step;
-          umma::mma(tmem + r * N_MAX, hi_desc + off, bd, id, tap > 0 ? 1u : first);
-          umma::mma(tmem + r * N_MAX, lo_desc + off, bd, id, 1u);
+          const uint64_t bd = w_desc + ((tap % 3u) * 6u + 2u - tap / 3u) * a.n;
+          umma::mma(tmem + r * a.n, hi_desc + off, bd, id, tap > 0 ? 1u : first);
+          umma::mma(tmem + r * a.n, lo_desc + off, bd, id, 1u);
         }
       }
       umma::commit(done0 + 8u * s);
@@ -487,10 +490,11 @@ constexpr uint32_t ws_threads() {
 }
 template <class S>
 __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_constant__ ConvArgs a) {
-  constexpr uint32_t STAGE = S::STAGE, A_BYTES = S::A_BYTES, CTRL = S::CTRL, N_MAX = S::N_MAX, ROWS = S::ROWS;
-  constexpr uint32_t NS = S::STAGES, ACC = ROWS * N_MAX, TMEM_COLS = 2u * ACC;
+  constexpr uint32_t STAGE = S::STAGE, A_BYTES = S::A_BYTES, CTRL = S::CTRL, ROWS = S::ROWS;
+  constexpr uint32_t NS = S::STAGES, ACC = ROWS * S::N_MAX, TMEM_COLS = 2u * ACC;
   constexpr uint32_t RAW_PLANE = S::RAW_PLANE, RAW_W = S::RAW_W;
   static_assert(TMEM_COLS <= 512u, "two accumulators in the TMEM of one SM");
+  static_assert((S::ROWS < 3u ? 2u : 3u) * S::N_MAX <= 256u, "columns of one MMA");
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   const uint32_t base = umma::smem_addr(smem);
@@ -562,8 +566,7 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
       }
     }
   } else if (tid == 32) {  // the MMAs
-    const uint32_t id = idesc_f16(128, a.n);
-    const uint32_t w_step = (2u * a.n * 16u) >> 4;
+    const uint32_t id1 = idesc_f16(128, a.n), id2 = idesc_f16(128, 2u * a.n), id3 = idesc_f16(128, 3u * a.n);
     uint32_t c = 0, i = 0, wph = 0;  // wph bit s: the parity of stage s's next widening
     for (uint32_t t = blockIdx.x; t < tiles && !*abort_flag; t += gridDim.x, ++i) {
       const uint32_t b = i & 1u, acc = tmem + b * ACC;
@@ -581,16 +584,29 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
         umma::fence_after();
         const uint64_t hi_desc = umma::desc(base + s * STAGE, A_PLANE, 128u);
         const uint64_t lo_desc = umma::desc(base + s * STAGE + A_BYTES, A_PLANE, 128u);
-        const uint64_t w_desc = umma::desc(base + s * STAGE + 2u * A_BYTES, a.n * 16u, 128u);
-        const uint32_t first = k == 0 ? 0u : 1u;
+        const uint64_t w_desc = umma::desc(base + s * STAGE + 2u * A_BYTES, 3u * a.n * 16u, 128u);
+        // Patch row y meets output rows y - 2 .. y with taps ky = 2 .. 0, which
+        // lie side by side in the weights as the rows' accumulators do in TMEM:
+        // one MMA of up to 3 n columns for what three of n would read the same
+        // A operand for.  An output row still meets its taps in the order ky,
+        // kx, hi, lo, so its sums are the same bits.
 #pragma unroll
-        for (uint32_t r = 0; r < ROWS; ++r) {
+        for (uint32_t y = 0; y < ROWS + 2u; ++y) {
+          const uint32_t r0 = y < 2u ? 0u : y - 2u, r1 = y < ROWS ? y : ROWS - 1u, rows = r1 - r0 + 1u;
+          const uint32_t id = rows == 1u ? id1 : (rows == 2u ? id2 : id3);
+          const uint32_t d = acc + r0 * a.n, w_row = (2u - (y - r0)) * a.n;
 #pragma unroll
-          for (uint32_t tap = 0; tap < 9; ++tap) {
-            const uint32_t off = ((r + tap / 3u) * 2u * A_PLANE + (tap % 3u) * 16u) / 16u;
-            const uint64_t bd = w_desc + tap * w_step;
-            umma::mma(acc + r * N_MAX, hi_desc + off, bd, id, tap > 0 ? 1u : first);
-            umma::mma(acc + r * N_MAX, lo_desc + off, bd, id, 1u);
+          for (uint32_t kx = 0; kx < 3u; ++kx) {
+            const uint32_t off = (y * 2u * A_PLANE + kx * 16u) / 16u;
+            const uint64_t bd = w_desc + kx * 6u * a.n + w_row;
+            if (kx == 0u && k == 0u && y < ROWS) {
+              // row y's first product overwrites its accumulator
+              if (rows > 1u) umma::mma(d, hi_desc + off, bd, rows == 2u ? id1 : id2, 1u);
+              umma::mma(acc + y * a.n, hi_desc + off, w_desc + 2u * a.n, id1, 0u);
+            } else {
+              umma::mma(d, hi_desc + off, bd, id, 1u);
+            }
+            umma::mma(d, lo_desc + off, bd, id, 1u);
           }
         }
         umma::commit(empty0 + 8u * s);
