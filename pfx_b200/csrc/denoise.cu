@@ -304,57 +304,74 @@ __device__ __forceinline__ void store_split8(uint16_t* hi, uint16_t* lo, size_t 
 // takes the max of its row pair in the thread and of the neighbouring lane
 // (max pooling after ReLU = ReLU after max pooling); the result is written as
 // its hi/lo planes, four times over (2x2) when the output is stored upsampled.
+// `part` of `parts` warps per lane quarter takes every parts-th piece (a row
+// pair's 16 columns).  Both rows' columns of the next piece are on their way
+// while a piece is worked on.
 template <class S>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, uint32_t warp, uint32_t lane,
-                                              uint32_t x0, uint32_t y0) {
+                                              uint32_t x0, uint32_t y0, uint32_t part, uint32_t parts) {
   const uint32_t x = x0 + warp * 32u + lane;
-  const uint32_t G = a.n >> 3;
-#pragma unroll 1
-  for (uint32_t r0 = 0; r0 < S::ROWS; r0 += 2u) {
-#pragma unroll 1
-    for (uint32_t j = 0; j < a.n; j += 16u) {
-      float v0[16], v1[16];
-      umma::ld16(umma::taddr(tmem, warp * 32u, r0 * a.n + j), v0);
-      umma::ld16(umma::taddr(tmem, warp * 32u, (r0 + 1u) * a.n + j), v1);
-      float b[16];
+  const uint32_t G = a.n >> 3, groups = a.n >> 4, pieces = (S::ROWS / 2u) * groups;
+  uint32_t q[2][2][16];  // [ping-pong][row]
+  auto start = [&](uint32_t piece, uint32_t (&r)[2][16]) {
+    const uint32_t at = umma::taddr(tmem, warp * 32u, (piece / groups) * 2u * a.n + (piece % groups) * 16u);
+    umma::ld16_start(at, r[0]);
+    umma::ld16_start(at + a.n, r[1]);
+  };
+  auto finish = [&](uint32_t piece, const uint32_t (&r)[2][16]) {
+    const uint32_t r0 = (piece / groups) * 2u, j = (piece % groups) * 16u;
+    float b[16];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) b[c] = __ldg(a.bias + j + c);
-      if (a.pool) {
-        float m[16];
+    for (int c = 0; c < 4; ++c)
+      reinterpret_cast<float4*>(b)[c] = __ldg(reinterpret_cast<const float4*>(a.bias + j) + c);
+    if (a.pool) {
+      float m[16];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          m[c] = fmaxf(v0[c], v1[c]);
-          m[c] = fmaxf(m[c], __shfl_xor_sync(0xffffffffu, m[c], 1));
-          m[c] = fmaxf(m[c] + b[c], 0.0f);
-        }
-        const uint32_t oy = (y0 + r0) >> 1, ox = x >> 1, OH = a.H >> 1, OW = a.W >> 1;
-        if ((lane & 1u) == 0u && oy < OH && ox < OW) {
-          store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3)) * OW + ox) * 8u, m);
-          store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3) + 1u) * OW + ox) * 8u, m + 8);
-        }
-      } else {
+      for (int c = 0; c < 16; ++c) {
+        m[c] = fmaxf(__uint_as_float(r[0][c]), __uint_as_float(r[1][c]));
+        m[c] = fmaxf(m[c], __shfl_xor_sync(0xffffffffu, m[c], 1));
+        m[c] = fmaxf(m[c] + b[c], 0.0f);
+      }
+      const uint32_t oy = (y0 + r0) >> 1, ox = x >> 1, OH = a.H >> 1, OW = a.W >> 1;
+      if ((lane & 1u) == 0u && oy < OH && ox < OW) {
+        store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3)) * OW + ox) * 8u, m);
+        store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3) + 1u) * OW + ox) * 8u, m + 8);
+      }
+    } else {
 #pragma unroll
-        for (uint32_t rr = 0; rr < 2; ++rr) {
-          const uint32_t y = y0 + r0 + rr;
-          float v[16];
+      for (uint32_t rr = 0; rr < 2; ++rr) {
+        const uint32_t y = y0 + r0 + rr;
+        float v[16];
 #pragma unroll
-          for (int c = 0; c < 16; ++c) v[c] = fmaxf((rr ? v1[c] : v0[c]) + b[c], 0.0f);
-          if (y < a.H && x < a.W) {
-            if (!a.up) {
-              store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3)) * a.W + x) * 8u, v);
-              store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3) + 1u) * a.W + x) * 8u, v + 8);
-            } else {
-              const uint32_t W2 = 2u * a.W;
+        for (int c = 0; c < 16; ++c) v[c] = fmaxf(__uint_as_float(r[rr][c]) + b[c], 0.0f);
+        if (y < a.H && x < a.W) {
+          if (!a.up) {
+            store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3)) * a.W + x) * 8u, v);
+            store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3) + 1u) * a.W + x) * 8u, v + 8);
+          } else {
+            const uint32_t W2 = 2u * a.W;
 #pragma unroll
-              for (uint32_t q = 0; q < 4; ++q) {
-                const size_t Y = 2u * y + (q >> 1), X = 2u * x + (q & 1u);
-                store_split8(a.dst_hi, a.dst_lo, ((Y * G + (j >> 3)) * W2 + X) * 8u, v);
-                store_split8(a.dst_hi, a.dst_lo, ((Y * G + (j >> 3) + 1u) * W2 + X) * 8u, v + 8);
-              }
+            for (uint32_t k = 0; k < 4; ++k) {
+              const size_t Y = 2u * y + (k >> 1), X = 2u * x + (k & 1u);
+              store_split8(a.dst_hi, a.dst_lo, ((Y * G + (j >> 3)) * W2 + X) * 8u, v);
+              store_split8(a.dst_hi, a.dst_lo, ((Y * G + (j >> 3) + 1u) * W2 + X) * 8u, v + 8);
             }
           }
         }
       }
+    }
+  };
+  if (part < pieces) start(part, q[0]);
+#pragma unroll 1
+  for (uint32_t piece = part; piece < pieces; piece += 2u * parts) {
+#pragma unroll
+    for (uint32_t h = 0; h < 2u; ++h) {
+      const uint32_t at = piece + h * parts;
+      if (at >= pieces) break;
+      umma::ld16_wait(q[h][0]);
+      umma::ld16_wait(q[h][1]);
+      if (at + parts < pieces) start(at + parts, q[h ^ 1u]);
+      finish(at, q[h]);
     }
   }
 }
@@ -462,7 +479,7 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
   if (late || !drained) {
     if (tid == 0) atomicOr(a.error, (late ? ERR_CONV_WAIT : 0u) | (drained ? 0u : ERR_CONV_DRAIN));
   } else {
-    conv_epilogue<S>(a, tmem, warp, lane, x0, y0);
+    conv_epilogue<S>(a, tmem, warp, lane, x0, y0, 0u, 1u);
   }
   umma::fence_before();
   __syncthreads();
@@ -484,9 +501,14 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
 // then release the raw buffer (`raw empty`) and tell the MMA lane (the
 // stage's `widened` barrier).  The stage's own `full` barrier then counts the
 // weights alone.  Waits are bounded as in k_conv.
+#ifndef WS_EPI
+#define WS_EPI 2
+#endif
+constexpr uint32_t WS_PARTS = WS_EPI;                       // epilogue warps per TMEM lane quarter
+constexpr uint32_t WS_WIDEN = 2u + 4u * WS_PARTS;           // the first widening warp
 template <class S>
 constexpr uint32_t ws_threads() {
-  return S::EXPAND ? 320u : 192u;
+  return (WS_WIDEN + (S::EXPAND ? 4u : 0u)) * 32u;
 }
 template <class S>
 __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_constant__ ConvArgs a) {
@@ -516,7 +538,7 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
     }
     for (uint32_t b = 0; b < 2u; ++b) {
       umma::mbar_init(accf0 + 8u * b, 1);
-      umma::mbar_init(acce0 + 8u * b, 4);
+      umma::mbar_init(acce0 + 8u * b, 4u * WS_PARTS);
     }
     for (uint32_t j = 0; j < RAWS; ++j) {
       umma::mbar_init(raw_full0 + 8u * j, 1);
@@ -615,7 +637,7 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
       if (*abort_flag) break;
       umma::commit(accf0 + 8u * b);
     }
-  } else if (warp >= 2u && warp < 6u) {  // the epilogue
+  } else if (warp >= 2u && warp < WS_WIDEN) {  // the epilogue
     const uint32_t quarter = warp & 3u;
     uint32_t i = 0;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
@@ -626,19 +648,28 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
         break;
       }
       umma::fence_after();
-      conv_epilogue<S>(a, tmem + b * ACC, quarter, lane, (t % gx) * CONV_PIX, (t / gx) * ROWS);
+      conv_epilogue<S>(a, tmem + b * ACC, quarter, lane, (t % gx) * CONV_PIX, (t / gx) * ROWS, (warp - 2u) >> 2,
+                       WS_PARTS);
       umma::fence_before();
       __syncwarp();
       if (lane == 0) umma::mbar_arrive(acce0 + 8u * b);
     }
-  } else if (S::EXPAND && warp >= 6u && half0) {  // the widening of a half-size first source
-    constexpr uint32_t ITEMS = 2u * S::PATCH_ROWS * 2u * PATCH_W;  // planes x rows x groups x pixels
-    const uint32_t e = tid - 192u;
+  } else if (S::EXPAND && warp >= WS_WIDEN && half0) {  // the widening of a half-size first source
+    // Tiles start at even pixels and rows, so patch pixel p reads raw pixel
+    // (p + 1) / 2 and patch row r raw row (r + 1) / 2: a thread takes pixel e
+    // of every row, group and plane, the first threads pixels 128 and 129 too,
+    // at offsets known at compile time.
+    static_assert(ROWS % 2u == 0u && CONV_PIX % 2u == 0u, "tiles start at even pixels");
+    constexpr uint32_t LINES = 2u * S::PATCH_ROWS * 2u;  // planes x rows x groups
+    const uint32_t e = tid - WS_WIDEN * 32u;
+    auto line = [&](uint32_t k, uint32_t& from, uint32_t& to) {  // k = (plane x rows + r) x 2 + group
+      const uint32_t grp = k & 1u, r = (k >> 1) % S::PATCH_ROWS, plane = (k >> 1) / S::PATCH_ROWS;
+      from = plane * RAW_PLANE + (((r + 1u) >> 1) * 2u + grp) * RAW_W * 16u;
+      to = plane * A_BYTES + (r * 2u + grp) * A_PLANE;
+    };
     uint32_t c = 0, u = 0;
     bool stop = false;
     for (uint32_t t = blockIdx.x; t < tiles && !stop; t += gridDim.x) {
-      const int x0 = (int)((t % gx) * CONV_PIX), y0 = (int)((t / gx) * ROWS);
-      const int xl = (x0 - 1) >> 1, yl = (y0 - 1) >> 1;  // the raw buffer's first pixel and row
       for (uint32_t k = 0; k < chunks; ++k, ++c) {
         if (k >= chunks0) continue;
         const uint32_t s = c % NS, j = u % RAWS;
@@ -650,12 +681,19 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
         }
         uint8_t* st = smem + s * STAGE;
         const uint8_t* raw = smem + S::RAW_AT + j * 2u * RAW_PLANE;
-        for (uint32_t item = e; item < ITEMS; item += 128u) {
-          const uint32_t p = item % PATCH_W, rest = item / PATCH_W;  // rest = (plane x rows + r) x 2 + group
-          const uint32_t grp = rest & 1u, r = (rest >> 1) % S::PATCH_ROWS, plane = (rest >> 1) / S::PATCH_ROWS;
-          const uint32_t rl = (uint32_t)(((y0 - 1 + (int)r) >> 1) - yl), pl = (uint32_t)(((x0 - 1 + (int)p) >> 1) - xl);
-          const uint4 v = *reinterpret_cast<const uint4*>(raw + plane * RAW_PLANE + ((rl * 2u + grp) * RAW_W + pl) * 16u);
-          *reinterpret_cast<uint4*>(st + plane * A_BYTES + (r * 2u + grp) * A_PLANE + p * 16u) = v;
+        const uint8_t* from_e = raw + ((e + 1u) >> 1) * 16u;
+        uint8_t* to_e = st + e * 16u;
+#pragma unroll
+        for (uint32_t l = 0; l < LINES; ++l) {
+          uint32_t from, to;
+          line(l, from, to);
+          *reinterpret_cast<uint4*>(to_e + to) = *reinterpret_cast<const uint4*>(from_e + from);
+        }
+        if (e < 2u * LINES) {
+          const uint32_t p = CONV_PIX + (e & 1u);
+          uint32_t from, to;
+          line(e >> 1, from, to);
+          *reinterpret_cast<uint4*>(st + to + p * 16u) = *reinterpret_cast<const uint4*>(raw + from + ((p + 1u) >> 1) * 16u);
         }
         umma::fence_async_smem();
         __syncwarp();
