@@ -181,8 +181,15 @@ namespace {
 __host__ __device__ constexpr uint32_t div_ceil(uint32_t a, uint32_t b) { return (a + b - 1u) / b; }
 
 constexpr uint32_t CONV_THREADS = 128;               // 4 warps: the epilogue by TMEM lane quarter
-constexpr uint32_t CONV_PIX = 128;                   // pixels per output row (M of the MMA)
-constexpr uint32_t PATCH_W = CONV_PIX + 2;           // staged pixels per input row
+// A tile is 126 output pixels wide and stages the 128 input pixels they need: a
+// row of a plane is then 2048 contiguous bytes, the 256 8-byte elements that
+// one row of a tensor copy may have.  (128 output pixels and 130 staged ones, as
+// rows of 16 bytes each, cost the copy engine a row of its box for every pixel:
+// the 4K frame 5.70 ms, 4.87 now.)  The MMA's rows 126 and 127 read up to two pixels into the next
+// plane for the later taps; what they yield is dropped.
+constexpr uint32_t CONV_PIX = 126;
+constexpr uint32_t PATCH_W = CONV_PIX + 2;           // staged pixels per input row, M of the MMA
+static_assert(PATCH_W == 128u, "M of the MMA");
 constexpr uint32_t A_PLANE = PATCH_W * 16u;          // bytes of one (row, group of 8 channels) plane
 
 // The shape of a conv CTA: ROWS output rows (one TMEM accumulator each, NMAX
@@ -218,11 +225,11 @@ template <uint32_t ROWS_, uint32_t NMAX_, uint32_t STAGES_, uint32_t CTAS_, bool
 struct ConvShape {
   static constexpr uint32_t ROWS = ROWS_, N_MAX = NMAX_, STAGES = STAGES_, CTAS = CTAS_;
   // EXPAND (persistent kernel only): a first source stored at half size is
-  // copied into one of RAWS raw buffers of ROWS / 2 + 2 rows x 66 pixels and
+  // copied into one of RAWS raw buffers of ROWS / 2 + 2 rows x 65 pixels and
   // widened 2x2 into the stage by four more warps.
   static constexpr bool EXPAND = EXPAND_;
   static constexpr uint32_t RAWS = RAWS_;
-  static constexpr uint32_t RAW_ROWS = ROWS / 2u + 2u, RAW_W = CONV_PIX / 2u + 2u;
+  static constexpr uint32_t RAW_ROWS = ROWS / 2u + 2u, RAW_W = PATCH_W / 2u + 1u;
   static constexpr uint32_t RAW_BOX = RAW_ROWS * 2u * RAW_W * 16u;   // one half (hi or lo) as copied
   static constexpr uint32_t RAW_PLANE = (RAW_BOX + 127u) / 128u * 128u;  // its place in shared memory
   static constexpr uint32_t RAW = EXPAND ? RAWS * 2u * RAW_PLANE : 0u;
@@ -310,7 +317,8 @@ __device__ __forceinline__ void store_split8(uint16_t* hi, uint16_t* lo, size_t 
 template <class S>
 __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, uint32_t warp, uint32_t lane,
                                               uint32_t x0, uint32_t y0, uint32_t part, uint32_t parts) {
-  const uint32_t x = x0 + warp * 32u + lane;
+  const uint32_t row = warp * 32u + lane, x = x0 + row;
+  const bool kept = row < CONV_PIX;  // rows 126 and 127 are no pixels of this tile
   const uint32_t G = a.n >> 3, groups = a.n >> 4, pieces = (S::ROWS / 2u) * groups;
   uint32_t q[2][2][16];  // [ping-pong][row]
   auto start = [&](uint32_t piece, uint32_t (&r)[2][16]) {
@@ -333,7 +341,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, 
         m[c] = fmaxf(m[c] + b[c], 0.0f);
       }
       const uint32_t oy = (y0 + r0) >> 1, ox = x >> 1, OH = a.H >> 1, OW = a.W >> 1;
-      if ((lane & 1u) == 0u && oy < OH && ox < OW) {
+      if ((lane & 1u) == 0u && kept && oy < OH && ox < OW) {
         store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3)) * OW + ox) * 8u, m);
         store_split8(a.dst_hi, a.dst_lo, (((size_t)oy * G + (j >> 3) + 1u) * OW + ox) * 8u, m + 8);
       }
@@ -344,7 +352,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, 
         float v[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) v[c] = fmaxf(__uint_as_float(r[rr][c]) + b[c], 0.0f);
-        if (y < a.H && x < a.W) {
+        if (kept && y < a.H && x < a.W) {
           if (!a.up) {
             store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3)) * a.W + x) * 8u, v);
             store_split8(a.dst_hi, a.dst_lo, (((size_t)y * G + (j >> 3) + 1u) * a.W + x) * 8u, v + 8);
@@ -377,9 +385,9 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t tmem, 
 }
 
 // One 3x3 convolution (+ bias, ReLU, and 2x2 max pooling when a.pool) of a
-// tile of ROWS rows x 128 pixels.  Grid: (ceil(W / 128), ceil(H / ROWS)).
+// tile of ROWS rows x 126 pixels.  Grid: (ceil(W / 126), ceil(H / ROWS)).
 // Lane 0 of warp 0 copies each chunk of 16 input channels into a stage: the
-// hi and lo planes' boxes of 8 halves x 130 pixels x 2 groups x (ROWS + 2)
+// hi and lo planes' boxes of 128 pixels x 2 groups x (ROWS + 2)
 // rows from the source's tensor maps (zeros outside the tensor: the
 // convolution's padding), and the chunk's weights by a bulk copy, all on the
 // stage's `full` barrier; lane 0 of warp 1 issues the chunk's MMAs once it is
@@ -426,8 +434,8 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
       umma::mbar_expect_tx(full, 2u * A_BYTES + wbytes);
       const bool first = k < chunks0;
       const int g = (int)(2u * (first ? k : k - chunks0));
-      umma::tensor_load_4d(st, first ? &a.a0_hi : &a.a1_hi, 0, (int)x0 - 1, g, (int)y0 - 1, full);
-      umma::tensor_load_4d(st + A_BYTES, first ? &a.a0_lo : &a.a1_lo, 0, (int)x0 - 1, g, (int)y0 - 1, full);
+      umma::tensor_load_3d(st, first ? &a.a0_hi : &a.a1_hi, 2 * ((int)x0 - 1), g, (int)y0 - 1, full);
+      umma::tensor_load_3d(st + A_BYTES, first ? &a.a0_lo : &a.a1_lo, 2 * ((int)x0 - 1), g, (int)y0 - 1, full);
       umma::bulk_load(st + 2u * A_BYTES, a.weights + (size_t)k * (wbytes / 2u), wbytes, full);
       loads = k + 1u;
     }
@@ -487,7 +495,7 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
 }
 
 // The persistent form of k_conv: one CTA per SM walks the layer's tiles
-// (tile t: pixels 128 (t % gx).., rows ROWS (t / gx)..) in steps of gridDim.x.
+// (tile t: pixels 126 (t % gx).., rows ROWS (t / gx)..) in steps of gridDim.x.
 // Lane 0 of warp 0 streams every tile's chunks through the NS-stage ring;
 // lane 0 of warp 1 issues each tile's MMAs into one of two TMEM accumulators
 // (tiles alternate) and commits it to the accumulator's `full` barrier; warps
@@ -575,13 +583,13 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
           umma::mbar_expect_tx(full, wbytes);
           umma::mbar_expect_tx(raw_full, 2u * S::RAW_BOX);
           const uint32_t raw = base + S::RAW_AT + j * 2u * RAW_PLANE;
-          umma::tensor_load_4d(raw, &a.a0_hi, 0, (x0 >> 1) - 1, g, (y0 >> 1) - 1, raw_full);
-          umma::tensor_load_4d(raw + RAW_PLANE, &a.a0_lo, 0, (x0 >> 1) - 1, g, (y0 >> 1) - 1, raw_full);
+          umma::tensor_load_3d(raw, &a.a0_hi, x0 - 2, g, (y0 >> 1) - 1, raw_full);
+          umma::tensor_load_3d(raw + RAW_PLANE, &a.a0_lo, x0 - 2, g, (y0 >> 1) - 1, raw_full);
           counts[2] = ++u;
         } else {
           umma::mbar_expect_tx(full, 2u * A_BYTES + wbytes);
-          umma::tensor_load_4d(st, first ? &a.a0_hi : &a.a1_hi, 0, x0 - 1, g, y0 - 1, full);
-          umma::tensor_load_4d(st + A_BYTES, first ? &a.a0_lo : &a.a1_lo, 0, x0 - 1, g, y0 - 1, full);
+          umma::tensor_load_3d(st, first ? &a.a0_hi : &a.a1_hi, 2 * (x0 - 1), g, y0 - 1, full);
+          umma::tensor_load_3d(st + A_BYTES, first ? &a.a0_lo : &a.a1_lo, 2 * (x0 - 1), g, y0 - 1, full);
         }
         umma::bulk_load(st + 2u * A_BYTES, a.weights + (size_t)k * (wbytes / 2u), wbytes, full);
         counts[0] = c + 1u;
@@ -657,8 +665,7 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
   } else if (S::EXPAND && warp >= WS_WIDEN && half0) {  // the widening of a half-size first source
     // Tiles start at even pixels and rows, so patch pixel p reads raw pixel
     // (p + 1) / 2 and patch row r raw row (r + 1) / 2: a thread takes pixel e
-    // of every row, group and plane, the first threads pixels 128 and 129 too,
-    // at offsets known at compile time.
+    // of every row, group and plane, at offsets known at compile time.
     static_assert(ROWS % 2u == 0u && CONV_PIX % 2u == 0u, "tiles start at even pixels");
     constexpr uint32_t LINES = 2u * S::PATCH_ROWS * 2u;  // planes x rows x groups
     const uint32_t e = tid - WS_WIDEN * 32u;
@@ -688,12 +695,6 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
           uint32_t from, to;
           line(l, from, to);
           *reinterpret_cast<uint4*>(to_e + to) = *reinterpret_cast<const uint4*>(from_e + from);
-        }
-        if (e < 2u * LINES) {
-          const uint32_t p = CONV_PIX + (e & 1u);
-          uint32_t from, to;
-          line(e >> 1, from, to);
-          *reinterpret_cast<uint4*>(st + to + p * 16u) = *reinterpret_cast<const uint4*>(raw + from + ((p + 1u) >> 1) * 16u);
         }
         umma::fence_async_smem();
         __syncwarp();
@@ -1050,18 +1051,19 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
   return fn;
 }
 
-// The tensor map of one plane of a U-Net tensor ([H][C/8][W][8] halves) for
-// boxes of 8 halves x 130 pixels x 2 groups x `rows` rows.
+// The tensor map of one plane of a U-Net tensor ([H][C/8][W][8] halves), its
+// rows of W pixels as 2 W elements of 8 bytes, for boxes of 128 pixels x 2
+// groups x `rows` + 2 rows; of a half-size source, for the raw box that
+// k_conv_ws widens (65 pixels, rows / 2 + 2 rows).
 CUtensorMap plane_map(const uint16_t* plane, uint32_t H, uint32_t W, uint32_t C, uint32_t rows, bool half = false) {
   CUtensorMap m;
-  const cuuint64_t dims[4] = {8u, W, C / 8u, H};
-  const cuuint64_t strides[3] = {16u, (cuuint64_t)W * 16u, (cuuint64_t)(C / 8u) * W * 16u};
-  // a half-size source is read as the raw box that k_conv_ws widens: RAW_W pixels, rows / 2 + 2 rows
-  const cuuint32_t box[4] = {8u, half ? CONV_PIX / 2u + 2u : PATCH_W, 2u, half ? rows / 2u + 2u : rows + 2u};
-  const cuuint32_t elem[4] = {1u, 1u, 1u, 1u};
-  CUresult r = encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<uint16_t*>(plane), dims, strides, box,
+  const cuuint64_t dims[3] = {2u * (cuuint64_t)W, C / 8u, H};
+  const cuuint64_t strides[2] = {(cuuint64_t)W * 16u, (cuuint64_t)(C / 8u) * W * 16u};
+  const cuuint32_t box[3] = {half ? PATCH_W + 2u : 2u * PATCH_W, 2u, half ? rows / 2u + 2u : rows + 2u};
+  const cuuint32_t elem[3] = {1u, 1u, 1u};
+  CUresult r = encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, const_cast<uint16_t*>(plane), dims, strides, box,
                               elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw DeviceError("denoiser tensor map: error " + std::to_string((int)r));
   return m;
 }
