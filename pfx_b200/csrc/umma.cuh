@@ -167,5 +167,11 @@ __device__ __forceinline__ uint32_t taddr(uint32_t base, uint32_t lane, uint32_t
   return base + (lane << 16) + col;
 }
 
+// Programmatic dependent launch: lets the next kernel of the stream come in as
+// SMs have room (once every CTA of this grid has said so), and waits until the
+// kernels before this one are done and their writes visible.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace umma
 }  // namespace pfxt

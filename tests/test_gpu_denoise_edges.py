@@ -20,3 +20,4 @@ def test_tile_edges(gpu, h, w):
     want = D.denoise(color, albedo, normal, D.build_net(D.parse_tza(blob)))
     assert gap(out, want) <= TOL, gap(out, want)
     assert np.array_equal(out.view(np.uint32), den.denoise(color, albedo, normal).view(np.uint32))
+
