@@ -539,7 +539,13 @@ struct Walker {
 // 1.5 M rays 1100 -> 925 us, instanced closest and any 0.5 M rays 476 -> 355
 // and 518 -> 403 us.  32 resident warps (64 registers) beat 24, 28, 36 and 40.
 //
-// Order.  Children are visited in the reference's left-first order and a
+// Order.  An any-hit answer does not depend on it, and a blocker is mostly near:
+// the nearest child goes first (1.5 M shadow rays in the room 925 -> 523 us,
+// instanced 406 -> 359).  For a closest hit children are visited in the
+// reference's left-first order (nearest first took 973 instead of 1794 us on the
+// room's 2^21 rays, and the same hits on 1.26 billion rays, but 12 of 10,000 rays
+// aimed to within 1e-8 rad along a triangle's plane ended elsewhere: such a
+// triangle's distance is off by any amount, so its box tells nothing) and a
 // popped entry is checked again against the current distance, so the leaves
 // tested, their order and the distance at each are the reference's.  A lane
 // that reaches a leaf while other lanes of its warp still walk inner nodes
@@ -654,8 +660,9 @@ struct QuadWalker {
     return !(n > f) && n <= reach;
   }
 
-  // Opens the inner node at hand: tests its four children loosely; the first
-  // that passes is next, the others are pushed last first.
+  // Opens the inner node at hand: tests its four children loosely.  Closest hit:
+  // the first that passes is next, the others are pushed last first; any hit:
+  // the nearest is next.
   template <class Stack>
   __device__ __forceinline__ void open(const SceneView& s, Stack& st) {
     const char* p = reinterpret_cast<const char*>(s.quad + ref);
@@ -680,9 +687,14 @@ struct QuadWalker {
         const float entry = fmaxf(max3f(fminf(xl[k], xh[k]), fminf(yl[k], yh[k]), fminf(zl[k], zh[k])), 0.0f);
         const float exit = fminf(min3f(fmaxf(xl[k], xh[k]), fmaxf(yl[k], yh[k]), fmaxf(zl[k], zh[k])), hit.t);
         if (entry <= exit * LOOSE) {
-          if (next != REF_NONE) st.put(top++, next, next_near);
-          next = h ? (k ? c.w : c.z) : (k ? c.y : c.x);
-          next_near = entry;
+          const uint32_t child = h ? (k ? c.w : c.z) : (k ? c.y : c.x);
+          if (ANY && next != REF_NONE && entry >= next_near) {
+            st.put(top++, child, entry);
+          } else {
+            if (next != REF_NONE) st.put(top++, next, next_near);
+            next = child;
+            next_near = entry;
+          }
         }
       }
     }

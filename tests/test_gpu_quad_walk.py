@@ -64,6 +64,58 @@ def test_small_trees(gpu, count, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["doubled", "needles", "stacked", "grid", "mixed"])
+def test_ties_and_slivers(gpu, kind):
+    """Where the order of the walk could show: the same triangles twice, needles
+    seen edge on, coplanar overlapping quads, rays through shared corners and
+    edges, and all of it over six orders of magnitude."""
+    rng = np.random.default_rng(len(kind))
+    n = 400
+    v = rng.uniform(-4, 4, (n, 1, 3)) + rng.uniform(-1.0, 1.0, (n, 3, 3))
+    if kind == "doubled":
+        v = np.concatenate([v, v[::-1], v[:, [1, 2, 0]]])
+    if kind == "needles":
+        v[:, 2] = v[:, 0] + (v[:, 1] - v[:, 0]) * rng.uniform(0.2, 0.9, (n, 1)) + rng.normal(size=(n, 3)) * 1e-5
+    if kind == "stacked":
+        v = np.round(v)
+        v[:, :, 1] = (np.arange(n) % 4)[:, None]
+    if kind == "grid":
+        x, z = np.meshgrid(np.arange(-7, 7), np.arange(-7, 7))
+        a = np.stack([x, 0.25 * ((x + z) % 3), z], -1).reshape(-1, 3).astype(float)
+        v = np.concatenate([a[:, None] + np.array([[0, 0, 0], [1, 0, 0], [1, 0, 1]]),
+                            a[:, None] + np.array([[0, 0, 0], [1, 0, 1], [0, 0, 1]])])
+    if kind == "mixed":
+        v *= 10.0 ** rng.uniform(-3, 3, (n, 1, 1))
+    scene = SceneDesc(synth.triangles(v.astype(F32)), synth.material(), synth.look_at((0, 0, 10), (0, 0, 0), 45, 1.0))
+    trace = Trace(scene, Settings(), 8, 8)
+    ref = oracle.scene_buffers(scene, Settings())
+    m = 40_000
+    f = v.astype(F32)
+    o = rng.uniform(-8, 8, (m, 3)).astype(F32)
+    # at corners, at edges, at insides, and (every fourth) along the plane of a triangle
+    t = rng.integers(0, len(f), m)
+    w = rng.dirichlet((1, 1, 1), m).astype(F32)
+    w[::3] = np.eye(3, dtype=F32)[rng.integers(0, 3, len(w[::3]))]
+    w[1::3, 0] = 0.0
+    aim = np.einsum("ij,ijk->ik", w / w.sum(1, keepdims=True), f[t]).astype(F32)
+    o[::4] = (aim + (f[t, 0] - f[t, 1]) * rng.uniform(1, 3, (m, 1)).astype(F32))[::4]
+    d = (aim - o).astype(F32)
+    assert compare(trace, ref, make_rays(o, d, 1e20)) > m // 3
+    compare(trace, ref, make_rays(o, d, rng.uniform(0.5, 1.5, m).astype(F32)))
+
+
+@pytest.mark.gpu
+def test_coincident_instances(gpu):
+    """Instances placed on one another: hits tie across instances."""
+    w = synth.instanced_1080(target=2000)
+    w.scene.instances = np.concatenate([w.scene.instances, w.scene.instances[::-1], w.scene.instances[::3]])
+    trace = Trace(w.scene, w.settings, 8, 8)
+    ref = oracle.scene_buffers(w.scene, w.settings)
+    o, d = rays_for(np.random.default_rng(4), (-60, 0, -60), (60, 40, 60), 20000)
+    assert compare(trace, ref, make_rays(o, d, 1e20)) > 1000
+
+
+@pytest.mark.gpu
 def test_instances_with_every_ray_class(gpu):
     w = synth.instanced_1080(target=3000)
     trace = Trace(w.scene, w.settings, 8, 8)
