@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
   w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0, item = 0;
-  bool have = false, retired = false;
+  bool have = false, retired = (uint32_t)lane >= lanes_per_warp(n, gridDim.x * (THREADS / 32u));
   for (;;) {
     bool need = !have && !retired;
     unsigned m = __ballot_sync(FULL, need);

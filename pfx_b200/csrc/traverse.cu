@@ -12,6 +12,7 @@
 // phase together.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "kernels.h"
@@ -39,7 +40,7 @@ constexpr uint32_t RETRY = QuadWalker<true>::RETRY;
 // four-box walk cannot take are marked RETRY for k_trace_retry.
 template <int MODE>
 __global__ void __launch_bounds__(kThreads, TRACE_WARPS_PER_SM * 32 / kThreads) k_trace(SceneView s, const pfxt_ray* __restrict__ rays, uint32_t n,
-                                                    void* __restrict__ out, uint32_t* __restrict__ counter) {
+                                                    void* __restrict__ out, uint32_t* __restrict__ counter, uint32_t lanes) {
   constexpr bool ANY = MODE == 1;
   constexpr unsigned FULL = 0xffffffffu;
   QuadStack st;
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(kThreads, TRACE_WARPS_PER_SM * 32 / kThreads) 
   w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0;
-  bool have = false, retired = false;
+  bool have = false, retired = lane >= (int)lanes;
   for (;;) {
     bool need = !have && !retired;
     unsigned m = __ballot_sync(FULL, need);
@@ -208,11 +209,11 @@ cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* o
   if (n == 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
-  uint32_t need = (n + kThreads - 1) / kThreads;
-  uint32_t blocks = (uint32_t)persistent_blocks<MODE>();
-  if (need < blocks) blocks = need;
-  k_trace<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter);
-  k_trace_retry<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out);
+  const uint32_t most = (uint32_t)persistent_blocks<MODE>();
+  const uint32_t lanes = lanes_per_warp(n, most * (kThreads / 32));
+  const uint32_t blocks = std::min(most, (n + lanes * (kThreads / 32) - 1) / (lanes * (kThreads / 32)));
+  k_trace<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter, lanes);
+  k_trace_retry<MODE><<<std::min(most, (n + kThreads - 1) / kThreads), kThreads, 0, stream>>>(s, rays, n, out);
   return cudaGetLastError();
 }
 
