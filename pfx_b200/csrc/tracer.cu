@@ -319,7 +319,7 @@ __global__ void k_seed_counts(const __grid_constant__ Pass P) {
 // Before a bounce: empty the next ray queue and the shadow queue, rewind the
 // work counter of the extend kernel, and count the closest-hit queries of the
 // bounce (64-bit totals at counters[8..9] closest, [10..11] any hit).
-__global__ void k_reset(const __grid_constant__ Pass P,uint32_t cur) {
+__device__ __forceinline__ void reset_bounce(const Pass& P, uint32_t cur) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     P.w.counters[cur ^ 1u] = 0u;
     P.w.counters[2] = 0u;
@@ -339,6 +339,7 @@ __global__ void k_reset(const __grid_constant__ Pass P,uint32_t cur) {
     }
   }
 }
+__global__ void k_reset(const __grid_constant__ Pass P, uint32_t cur) { reset_bounce(P, cur); }
 
 // ------------------------------------------------------------------ sort
 // The shade queue grouped by the material of each path's hit (misses last),
@@ -461,14 +462,20 @@ __global__ void __launch_bounds__(256) k_sort_place(const __grid_constant__ Pass
   }
 }
 // Before the connect: rewind its work counter and take its own copy of the
-// shadow-queue count (the next bounce's k_reset may empty the queue count
-// while the connect still runs), and count the any-hit queries.
-__global__ void k_rewind(const __grid_constant__ Pass P) {
+// shadow-queue count (the next bounce empties the queue count while the connect
+// still runs), and count the any-hit queries.  NEXT: what k_reset does for the
+// next bounce (its queue is `cur`) in the same launch.
+template <bool NEXT>
+__global__ void k_rewind(const __grid_constant__ Pass P, uint32_t cur) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     P.w.counters[16] = 0u;
     P.w.counters[17] = P.w.counters[2];
     P.w.counters[14] = 0u;
     reinterpret_cast<unsigned long long*>(P.w.counters + 8)[1] += P.w.counters[2];
+  }
+  if (NEXT) {
+    __syncthreads();
+    reset_bounce(P, cur);
   }
 }
 
@@ -1180,11 +1187,15 @@ __device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i, uint32_t pixe
 // kinds of children, one loop body for both children) 1038 us and 7,200.
 // Blocks of 128 per SM: 6, 8, 10 and 12 gave a 1280 x 720 frame at 16 samples
 // 91.1, 90.6, 90.2 and 96.4 ms.
-__global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const __grid_constant__ Pass P, uint32_t k) {
+// `skip` draws of the pcg state are a black sky's, which adds nothing else.
+__global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const __grid_constant__ Pass P, uint32_t k,
+                                                                         uint32_t skip) {
   const uint32_t n = P.w.counters[12];
   const Specialise& sp = P.sp;
   const ShadeView& V = P.v;
-  for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < n; qi += gridDim.x * blockDim.x) {
+  const uint32_t warps = gridDim.x * (kThreads / 32u), lanes = lanes_per_warp(n, warps), lane = threadIdx.x & 31u;
+  if (lane >= lanes) return;
+  for (uint32_t qi = ((blockIdx.x * kThreads + threadIdx.x) >> 5) * lanes + lane; qi < n; qi += warps * lanes) {
     const uint32_t i = P.w.lit[qi];
     float4* record = P.w.surf + (size_t)i * 4u;
     const Pair g = load_pair(record);
@@ -1195,6 +1206,7 @@ __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const _
       start = sobol_z(V, sp, slot_rng(P, i, __float_as_uint(reinterpret_cast<const float*>(P.w.tr + 2u * i + 1u)[3])),
                       light_dim(k));
     } else {
+      for (uint32_t s = 0u; s < skip; ++s) state = pcg(state);
       start = random01(state);
       reinterpret_cast<float*>(P.w.tr + 2u * i)[3] = __uint_as_float(state);
     }
@@ -1548,14 +1560,18 @@ void launch_light_slots(const Pass& P, cudaStream_t st) {
   Grids& g = grids();
   const bool black_sky = P.v.sky_radiance[0] == 0.0f && P.v.sky_radiance[1] == 0.0f && P.v.sky_radiance[2] == 0.0f;
   if (P.f.sun_color[3] > 0.0f) k_light_slot<SLOT_SUN><<<g.slot[SLOT_SUN], kThreads, 0, st>>>(P, 0u);
-  if (P.v.sky_width != 0u && !(black_sky && P.sp.sobol))
+  // with nothing live between the two, the tree's descent takes the black sky's draws along
+  const bool tree = P.slots > 3u + P.v.looped;
+  const uint32_t skip =
+      black_sky && !P.sp.sobol && P.v.sky_width != 0u && tree && P.v.emitter_count == 0u && P.v.looped == 0u ? 2u : 0u;
+  if (P.v.sky_width != 0u && !(black_sky && P.sp.sobol) && skip == 0u)
     k_light_slot<SLOT_SKY><<<g.slot[SLOT_SKY], kThreads, 0, st>>>(P, 1u);
   if (P.v.emitter_count != 0u) k_light_slot<SLOT_EMITTER><<<g.slot[SLOT_EMITTER], kThreads, 0, st>>>(P, 2u);
   for (uint32_t s = 1u; s <= P.v.looped; ++s)
     k_light_slot<SLOT_LOOPED><<<g.slot[SLOT_LOOPED], kThreads, 0, st>>>(P, 2u + s);
-  if (P.slots > 3u + P.v.looped) {
+  if (tree) {
     const uint32_t k = 3u + P.v.looped;
-    k_tree_pick<<<g.tree_pick, kThreads, 0, st>>>(P, k);
+    k_tree_pick<<<g.tree_pick, kThreads, 0, st>>>(P, k, skip);
     k_light_slot<SLOT_TREE><<<g.slot[SLOT_TREE], kThreads, 0, st>>>(P, k);
   }
 }
@@ -1905,8 +1921,8 @@ void enqueue_pass(pfxt_trace& t, Pass& P, uint32_t count, bool deferred, uint32_
   k_collect<<<g.flat, 256, 0, st>>>(P, t.d_accum, t.d_mask);
   bool inferred = false;
   // A bounce's extend: empty the next queues, sort the rays (when chosen), walk.
-  auto extend = [&](const Pass& Q, uint32_t cur, cudaStream_t s) {
-    k_reset<<<1, 32, 0, s>>>(Q, cur);
+  auto extend = [&](const Pass& Q, uint32_t cur, cudaStream_t s, bool reset) {
+    if (reset) k_reset<<<1, 32, 0, s>>>(Q, cur);
     if (Q.ray_bins && Q.bounce > 0u) {
       k_sort_count<true><<<g.flat, 256, 0, s>>>(Q, cur);
       k_sort_place<true><<<g.flat, 256, 0, s>>>(Q, cur);
@@ -1934,7 +1950,7 @@ void enqueue_pass(pfxt_trace& t, Pass& P, uint32_t count, bool deferred, uint32_
       if (ahead && bounce > 0u)
         check(cudaStreamWaitEvent(st, t.ahead_join, 0), "extend join");
       else
-        extend(P, cur, st);
+        extend(P, cur, st, true);
       if (P.bins) {
         k_sort_count<false><<<g.flat, 256, 0, st>>>(P, cur);
         k_sort_place<false><<<g.flat, 256, 0, st>>>(P, cur);
@@ -1964,13 +1980,16 @@ void enqueue_pass(pfxt_trace& t, Pass& P, uint32_t count, bool deferred, uint32_
         inferred = true;
       }
       if (deferred) {
-        k_rewind<<<1, 32, 0, st>>>(P);
+        if (ahead && bounce < last)
+          k_rewind<true><<<1, 32, 0, st>>>(P, (bounce + 1u) & 1u);
+        else
+          k_rewind<false><<<1, 32, 0, st>>>(P, 0u);
         if (ahead && bounce < last) {
           Pass Q = P;
           Q.bounce = bounce + 1u;
           check(cudaEventRecord(t.ahead_fork, st), "extend fork");
           check(cudaStreamWaitEvent(t.ahead, t.ahead_fork, 0), "extend fork");
-          extend(Q, (bounce + 1u) & 1u, t.ahead);
+          extend(Q, (bounce + 1u) & 1u, t.ahead, false);
           check(cudaEventRecord(t.ahead_join, t.ahead), "extend join");
         }
         launch_trace_queue<true>(thread_select(t.trace_threads), t.short_stack, P, 0u, st);
