@@ -947,7 +947,11 @@ __device__ __forceinline__ float2 pick_importance(const PickRow* __restrict__ ro
 }
 
 // tree_pick on the PickRows: the same values bit for bit.
+// PAIR: this lane and its neighbour (lane ^ 1) run the same descent, the even
+// one evaluating every left child and the odd one every right child.
+template <bool PAIR>
 __device__ __forceinline__ float2 tree_pick_rows(const ShadeView& v, uint32_t rows, v3 p, v3 n, float start) {
+  const uint32_t odd = threadIdx.x & 1u;
   const PickRow* __restrict__ table = v.pick_rows;
   uint32_t at = f2u((float)v.looped + (float)v.tree);
   float rand = start, pdf = 1.0f;
@@ -973,12 +977,22 @@ __device__ __forceinline__ float2 tree_pick_rows(const ShadeView& v, uint32_t ro
     if (link >= rows) break;
     float2 l = make_float2(0.0f, 0.0f), r = l;
 #pragma unroll 1
-    for (uint32_t c = 0u; c < 2u; ++c) {  // one body for both children: the kernel is bound by issue and code
+    for (uint32_t c = PAIR ? odd : 0u, end = PAIR ? odd + 1u : 2u; c < end; ++c) {
+      // one body for both children: the kernel is bound by issue and code
       const float2 w = pick_importance(table, c ? link : left, p, n);
       if (c == 0u)
         l = w;
       else
         r = w;
+    }
+    if (PAIR) {
+      const unsigned both = 3u << (threadIdx.x & 30u);
+      const float2 mine = odd ? r : l;
+      const float2 other = make_float2(__shfl_xor_sync(both, mine.x, 1), __shfl_xor_sync(both, mine.y, 1));
+      if (odd)
+        l = other;
+      else
+        r = other;
     }
     const float total_max = l.x + r.x;
     if (total_max == 0.0f) return make_float2(0.0f, 0.0f);

@@ -1188,18 +1188,17 @@ __device__ __forceinline__ Rng slot_rng(const Pass& P, uint32_t i, uint32_t pixe
 // Blocks of 128 per SM: 6, 8, 10 and 12 gave a 1280 x 720 frame at 16 samples
 // 91.1, 90.6, 90.2 and 96.4 ms.
 // `skip` draws of the pcg state are a black sky's, which adds nothing else.
-__global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const __grid_constant__ Pass P, uint32_t k,
-                                                                         uint32_t skip) {
-  const uint32_t n = P.w.counters[12];
+template <bool PAIR>
+__device__ __forceinline__ void pick_paths(const Pass& P, uint32_t k, uint32_t skip, uint32_t n, uint32_t lanes,
+                                           uint32_t warps) {
   const Specialise& sp = P.sp;
   const ShadeView& V = P.v;
-  const uint32_t warps = gridDim.x * (kThreads / 32u), lanes = lanes_per_warp(n, warps), lane = threadIdx.x & 31u;
+  const uint32_t lane = (threadIdx.x & 31u) >> (PAIR ? 1u : 0u);
   if (lane >= lanes) return;
   for (uint32_t qi = ((blockIdx.x * kThreads + threadIdx.x) >> 5) * lanes + lane; qi < n; qi += warps * lanes) {
     const uint32_t i = P.w.lit[qi];
     float4* record = P.w.surf + (size_t)i * 4u;
     const Pair g = load_pair(record);
-    const float4 g0 = g.a, g1 = g.b;
     uint32_t state = __float_as_uint(reinterpret_cast<const float*>(P.w.tr + 2u * i)[3]);
     float start;
     if (sp.sobol) {
@@ -1208,11 +1207,29 @@ __global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const _
     } else {
       for (uint32_t s = 0u; s < skip; ++s) state = pcg(state);
       start = random01(state);
+      // both lanes of a pair have read the state before they write it (the same value)
+      if (PAIR) __syncwarp(3u << (threadIdx.x & 30u));
       reinterpret_cast<float*>(P.w.tr + 2u * i)[3] = __uint_as_float(state);
     }
-    *reinterpret_cast<float2*>(record + 3) =
-        tree_pick_rows(V, P.light_rows, mk3(g0.x, g0.y, g0.z), mk3(g1.x, g1.y, g1.z), start);
+    const float2 pick =
+        tree_pick_rows<PAIR>(V, P.light_rows, mk3(g.a.x, g.a.y, g.a.z), mk3(g.b.x, g.b.y, g.b.z), start);
+    if (!PAIR || (threadIdx.x & 1u) == 0u) *reinterpret_cast<float2*>(record + 3) = pick;
   }
+}
+__device__ __noinline__ void pick_pairs(const Pass& P, uint32_t k, uint32_t skip, uint32_t n, uint32_t lanes,
+                                        uint32_t warps) {
+  pick_paths<true>(P, k, skip, n, lanes, warps);
+}
+__global__ void __launch_bounds__(kThreads, PICK_MIN_BLOCKS) k_tree_pick(const __grid_constant__ Pass P, uint32_t k,
+                                                                         uint32_t skip) {
+  const uint32_t n = P.w.counters[12], warps = gridDim.x * (kThreads / 32u), lanes = lanes_per_warp(n, warps);
+  // Where half a warp's lanes would be idle, two lanes take a path: a descent's
+  // latency is one child a level instead of two (a 320 x 180 preview, 57,600
+  // paths: 1348 -> 1265 us).
+  if (lanes <= 16u)
+    pick_pairs(P, k, skip, n, lanes, warps);  // out of line, so that its registers are its own
+  else
+    pick_paths<false>(P, k, skip, n, lanes, warps);
 }
 
 // Slot k of kind KIND for every scattering path: the body of k_shade_lights'
