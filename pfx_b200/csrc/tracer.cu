@@ -1634,7 +1634,13 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
     }
     buffer = nullptr;
     held = 0;
-    check(cudaMalloc(&buffer, need), "wavefront path state");
+    const cudaError_t e = cudaMalloc(&buffer, need);
+    if (e != cudaSuccess) buffer = nullptr;
+    if (wide && e == cudaErrorMemoryAllocation) {  // another program took the memory meanwhile
+      cudaGetLastError();
+      return false;
+    }
+    check(e, "wavefront path state");
     held = need;
   }
   char* b = static_cast<char*>(buffer);
