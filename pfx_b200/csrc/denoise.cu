@@ -2,20 +2,22 @@
 // runs it (lib.rs, net.rs, tile.rs, process.wgsl, wgsl.rs), with the U-Net's
 // 3x3 convolutions as implicit GEMMs on the 5th-generation tensor cores.
 //
-// Layout.  A tensor of the U-Net is FP32, channels last, [y][x][C] with C
-// padded to a multiple of 16, at its level's size (the tile's size >> level).
-// A convolution is a GEMM per tile of R = 4 output rows x 128 pixels: M = the
-// 128 pixels of a row, N = the output channels, K = 9 taps x the input
-// channels, walked in chunks of 16 input channels.  For a chunk, the R + 2
-// input rows x 130 pixels (one pixel of border each side) are staged in shared
-// memory in the no-swizzle K-major canonical layout, pixel after pixel
-// (16 bytes = 8 channels per row of a core matrix), so the A operand of tap
-// (ky, kx) for output row r is the same bytes at a start address moved by
-// (r + ky) rows and kx pixels: no data moves per tap.  The chunk's weights
-// (9 taps x 16 channels x N) are one contiguous block, staged by one bulk
-// copy (TMA, no multicast).  One thread issues tcgen05.mma.kind::f16 (M =
-// 128, K = 16) into R accumulators in TMEM (columns 128 r), and the next
-// chunk is staged while those MMAs run (two stages).
+// Layout.  A tensor of the U-Net is two FP16 planes (hi and lo, below), each
+// [y][channel group of 8][x][8 halves] with C padded to a multiple of 16, at its
+// level's size (the tile's size >> level).  A convolution is a GEMM per tile of
+// ROWS output rows x 126 pixels: M = the 128 staged pixels of a row, N = the
+// output channels, K = 9 taps x the input channels, walked in chunks of 16
+// input channels.  For a chunk, the ROWS + 2 input rows x 128 pixels (one pixel
+// of border each side) are staged in shared memory in the no-swizzle K-major
+// canonical layout, pixel after pixel (16 bytes = 8 channels per row of a core
+// matrix), so the A operand of tap (ky, kx) for output row r is the same bytes
+// at a start address moved by (r + ky) rows and kx pixels: no data moves per
+// tap.  The chunk's weights (9 taps x 16 channels x N) are one contiguous
+// block, staged by one bulk copy (TMA, no multicast).  One thread issues
+// tcgen05.mma.kind::f16 (M = 128, K = 16).  An input row serves up to three
+// output rows, whose accumulators lie side by side in TMEM, so one MMA of up to
+// 3 N columns multiplies it by the weights of its three ky (conv_chunks).  The
+// next chunks are copied while those MMAs run.
 //
 // Precision.  The reference computes in FP32 (weights are FP16 in the blob,
 // exact in FP32).  Each staged activation is split into hi = fp16(a) and lo =
@@ -24,11 +26,12 @@
 // are exact, and the sums round in FP32 as the reference's do (in another
 // order).  Weights that are not exact in FP16 are refused.
 //
-// Epilogue.  tcgen05.ld per 16 columns, bias, ReLU; a pooling layer takes the
-// max of its two rows in the thread and of the neighbouring pixel's lane by
-// a shuffle (max pooling after ReLU = ReLU after max pooling).  Upsampling and
-// concatenation are in the staging: channels of the first source are read at
-// (y / 2, x / 2) of the half-size tensor, the skip source's at (y, x).
+// Epilogue.  tcgen05.ld per 16 columns, the next 16 under way while these are
+// worked on: bias, ReLU; a pooling layer takes the max of its two rows in the
+// thread and of the neighbouring pixel's lane by a shuffle (max pooling after
+// ReLU = ReLU after max pooling).  Upsampling and concatenation are in the
+// staging: an upsampled source is copied at its half size and widened 2x2 in
+// shared memory, the skip source is copied as it is.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_fp16.h>
@@ -198,7 +201,8 @@ constexpr uint32_t A_PLANE = PATCH_W * 16u;          // bytes of one (row, group
 // HBM) with the other's copies and MMAs, and more stages in one CTA overlap
 // only the copies; the persistent k_conv_ws overlaps all three in one CTA.
 // The 4K frame (two tiles of 2016x2160), forcing one shape wherever it fits
-// (the wide layers, above 64 channels, otherwise on Wide):
+// (the wide layers, above 64 channels, otherwise on Wide), with tiles of 128
+// pixels and one MMA per output row, tap and half:
 //  * k_conv, Tall:   8 rows, up to 64 channels, two stages, one CTA: 10.13 ms;
 //  * k_conv, Quad:   4 rows, up to 64 channels, three stages, one CTA: 11.08 ms;
 //  * k_conv, Wide:   4 rows, up to 128 channels, two stages, one CTA: 11.07 ms;
@@ -220,12 +224,15 @@ constexpr uint32_t A_PLANE = PATCH_W * 16u;          // bytes of one (row, group
 // rows no longer wait for the widening of the last).  Persist32 as 4 rows and
 // three stages instead: 6.66 ms against 6.54; as 6 rows and three stages
 // (384 of 512 TMEM columns): 6.62 ms, the same image bit for bit.
+// With the MMAs over up to three output rows 6.73 ms where the form before took
+// 7.22 (later boxes), with two epilogue warps a quarter 5.70, with tiles of 126
+// pixels 4.87, with each layer's set-up beside the layer before it 4.82.
 template <uint32_t ROWS_, uint32_t NMAX_, uint32_t STAGES_, uint32_t CTAS_, bool EXPAND_ = false,
           uint32_t RAWS_ = 1>
 struct ConvShape {
   static constexpr uint32_t ROWS = ROWS_, N_MAX = NMAX_, STAGES = STAGES_, CTAS = CTAS_;
   // EXPAND (persistent kernel only): a first source stored at half size is
-  // copied into one of RAWS raw buffers of ROWS / 2 + 2 rows x 65 pixels and
+  // copied into one of RAWS raw buffers of ROWS / 2 + 2 rows x RAW_W pixels and
   // widened 2x2 into the stage by four more warps.
   static constexpr bool EXPAND = EXPAND_;
   static constexpr uint32_t RAWS = RAWS_;
@@ -499,20 +506,17 @@ __global__ void __launch_bounds__(CONV_THREADS, S::CTAS) k_conv(const __grid_con
 // Lane 0 of warp 0 streams every tile's chunks through the NS-stage ring;
 // lane 0 of warp 1 issues each tile's MMAs into one of two TMEM accumulators
 // (tiles alternate) and commits it to the accumulator's `full` barrier; warps
-// 2-5 (TMEM lane quarters 2, 3, 0, 1) run the epilogue of one accumulator while
-// the MMAs of the next tile fill the other, and free it on its `empty`
-// barrier (one arrival per warp).  With an EXPAND shape and a first source
+// 2-9 (TMEM lane quarters 2, 3, 0, 1, twice: WS_PARTS) run the epilogue of one
+// accumulator while the MMAs of the next tile fill the other, and free it on its
+// `empty` barrier (one arrival per warp).  With an EXPAND shape and a first source
 // stored at half size (a.half0), that source's chunks are copied into a raw
-// buffer of RAW_ROWS x RAW_W pixels, and warps 6-9 widen it 2x2 into the
+// buffer of RAW_ROWS x RAW_W pixels, and warps 10-13 widen it 2x2 into the
 // stage (patch pixel p of row r reads raw pixel floor((x0 - 1 + p) / 2) -
 // floor((x0 - 1) / 2) of raw row floor((y0 - 1 + r) / 2) - floor((y0 - 1) / 2)),
 // then release the raw buffer (`raw empty`) and tell the MMA lane (the
 // stage's `widened` barrier).  The stage's own `full` barrier then counts the
 // weights alone.  Waits are bounded as in k_conv.
-#ifndef WS_EPI
-#define WS_EPI 2
-#endif
-constexpr uint32_t WS_PARTS = WS_EPI;                       // epilogue warps per TMEM lane quarter
+constexpr uint32_t WS_PARTS = 2u;                           // epilogue warps per TMEM lane quarter
 constexpr uint32_t WS_WIDEN = 2u + 4u * WS_PARTS;           // the first widening warp
 template <class S>
 constexpr uint32_t ws_threads() {

@@ -2,13 +2,13 @@
 //
 // Closest hit restates scene() (crates/trace/src/trace.wgsl:999-1075, with
 // tri_hit :780-804 and box_hit :453-468); any hit restates occluded()
-// (:1096-1168, tri_blocks :1076-1095).  Both walk the reference's tree in the
-// reference's order (left child first, right child when the left subtree is
-// done), test the same fp32 boxes with the same slab arithmetic (the quotients
+// (:1096-1168, tri_blocks :1076-1095).  Both walk the reference's tree, the
+// closest hit in the reference's order (left child first, right child when the
+// left subtree is done).  What decides a hit is tested as the reference tests
+// it: the same fp32 boxes with the same slab arithmetic (the quotients
 // (lo - o)/d are correctly rounded, so they equal the reference's divisions
-// bit for bit), and run the same Moller-Trumbore test
-// with the same operation order, so the hit slot, record and distance are
-// bit-identical to the CPU oracle's.  Clip planes, cutouts, alpha, sprites,
+// bit for bit) and the same Moller-Trumbore test with the same operation order,
+// so the hit slot, record and distance are bit-identical to the CPU oracle's.  Clip planes, cutouts, alpha, sprites,
 // motion and analytic shapes are outside this library's scope; the scenes it
 // accepts have none.
 //
@@ -545,8 +545,8 @@ struct Walker {
 // a whole sector of an axis, four loads a node (with six 16-byte loads of the
 // planes that the ray's signs pick: 1897 and 1048 us instead of 1797 and 925).
 // Start to now, one B200: room closest 2^21 rays 2646 -> 1797 us, room any
-// 1.5 M rays 1100 -> 925 us, instanced closest and any 0.5 M rays 476 -> 355
-// and 518 -> 403 us.  32 resident warps (64 registers) beat 24, 28, 36 and 40.
+// 1.5 M rays 1100 -> 925 us (523 by the order below), instanced closest and any
+// 0.5 M rays 476 -> 355 and 518 -> 403 us (359).  32 resident warps (64 registers) beat 24, 28, 36 and 40.
 //
 // Order.  An any-hit answer does not depend on it, and a blocker is mostly near:
 // the nearest child goes first (1.5 M shadow rays in the room 925 -> 523 us,
