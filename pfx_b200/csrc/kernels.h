@@ -25,5 +25,8 @@ cudaError_t launch_counts(const SceneView& s, const pfxt_ray* rays, uint32_t n, 
                           cudaStream_t stream);
 // The four-box nodes of `n` two-box nodes, by the same index.
 cudaError_t launch_collapse(const WideNode* wide, uint32_t n, QuadNode* quad, cudaStream_t stream);
+// The traversal triangles of `n` triangle records; leaf_of as in TraversalLayout.
+cudaError_t launch_lay_triangles(const GpuTriangle* records, const uint32_t* leaf_of, uint32_t n,
+                                 const WideNode* wide, TravTri* out, cudaStream_t stream);
 
 }  // namespace pfxt

@@ -46,12 +46,11 @@ struct Builder {
   uint64_t reach = 0;  // running maximum while one subtree is laid out
 
   // The slot base of the subtree being laid out (0: the top level's own
-  // leaves), the base each pseudo-parent's subtree was laid out with, and
-  // which slots have their leaf's box.  Scene builds put a slot in one leaf;
-  // buffers that do not are walked with the two-box nodes alone (`unboxed`).
+  // leaves) and the base each pseudo-parent's subtree was laid out with.  Scene
+  // builds put a slot in one leaf; buffers that do not are walked with the
+  // two-box nodes alone (`unboxed`).
   uint32_t base = 0;
   std::unordered_map<uint32_t, uint32_t> base_of;
-  std::vector<uint8_t> boxed;
   bool unboxed = false;
   // Entries the four-box walk's stack needs (the buffers' own max_depth is the
   // caller's word, and the two-box walk's): below the child laid out last as one
@@ -79,23 +78,25 @@ struct Builder {
     return most;
   }
 
-  void box_leaf(const GpuNode& n) {
+  // The leaf `at` (wide node << 1 | child, whose box the wide node has already).
+  void box_leaf(const GpuNode& n, uint32_t at) {
     const uint64_t first = (uint64_t)base + n.first;
     if (first + n.count > tri_count) return;  // refused by the reach check
     for (uint64_t i = first; i < first + n.count; ++i) {
-      TravTri& t = out.tris[i];
-      if (boxed[i] && (memcmp(t.lo, n.lo, 12) != 0 || memcmp(t.hi, n.hi, 12) != 0)) unboxed = true;
-      memcpy(t.lo, n.lo, 12);
-      memcpy(t.hi, n.hi, 12);
-      boxed[i] = 1u;
+      const uint32_t earlier = out.leaf_of[i];
+      if (earlier != REF_NONE) {
+        const float* f = &out.wide[earlier >> 1].b0[0] + 6u * (earlier & 1u);
+        if (memcmp(f, n.lo, 12) != 0 || memcmp(f + 3, n.hi, 12) != 0) unboxed = true;
+      }
+      out.leaf_of[i] = at;
     }
   }
 
-  uint32_t leaf_ref(const GpuNode& n) {
+  uint32_t leaf_ref(const GpuNode& n, uint32_t at) {
     if (n.count == 0 || n.count > 16) throw Invalid("BVH leaf holds more than 16 triangles");
     if (n.first > LEAF_FIRST_MASK) throw Invalid("BVH leaf offset exceeds the traversal encoding");
     reach = std::max<uint64_t>(reach, (uint64_t)n.first + n.count);
-    box_leaf(n);
+    box_leaf(n, at);
     return REF_LEAF | ((n.count - 1u) << LEAF_FIRST_BITS) | n.first;
   }
 
@@ -142,13 +143,13 @@ struct Builder {
     return REF_INST | index;
   }
 
-  // Reference of child node `i` as seen from its parent.
-  uint32_t child_ref(uint32_t i) {
+  // Reference of child node `i` as seen from its parent, which holds it at `at`.
+  uint32_t child_ref(uint32_t i, uint32_t at) {
     const GpuNode& n = nodes[i];
     if (n.pad[0] == INSTANCE_LEAF) return inst_ref(n);
     if (n.count == 0) return wide_of(i);
     need = Need{};
-    return leaf_ref(n);
+    return leaf_ref(n, at);
   }
 
   uint32_t pseudo(uint32_t root) {
@@ -162,7 +163,8 @@ struct Builder {
     reach = 0;
     WideNode node{};
     set_box(node, 0, nodes[root]);
-    node.child[0] = child_ref(root);
+    out.wide[w] = node;
+    node.child[0] = child_ref(root, w << 1);
     node.child[1] = REF_NONE;
     out.wide[w] = node;
     need_of[w] = need.whole;
@@ -181,9 +183,10 @@ struct Builder {
     WideNode node{};
     set_box(node, 0, nodes[left]);
     set_box(node, 1, nodes[right]);
-    node.child[0] = child_ref(left);
+    out.wide[w] = node;
+    node.child[0] = child_ref(left, w << 1);
     const Need l = need;
-    node.child[1] = child_ref(right);
+    node.child[1] = child_ref(right, w << 1 | 1u);
     const Need r = need;
     need.whole = quad_need(l, r);
     need.child[0] = l.whole;
@@ -204,8 +207,7 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
   builder.surface_count = b.surfaces_bytes / sizeof(GpuSurface);
   builder.tri_count = b.triangles_bytes / sizeof(GpuTriangle);
   if (b.triangle_count != builder.tri_count) throw Invalid("triangle count does not match the triangle buffer");
-  builder.out.tris.resize(builder.tri_count);
-  builder.boxed.assign(builder.tri_count, 0u);
+  builder.out.leaf_of.assign(builder.tri_count, REF_NONE);
   if (builder.node_count > 0 && b.triangle_count > 0) {
     builder.out.wide.reserve(builder.node_count / 2 + 16);
     builder.out.root = builder.pseudo(0);
@@ -229,17 +231,6 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
     }
     for (int k = 0; k < 3; ++k)
       if (!(f[k] <= f[3 + k]) || !(f[6 + k] <= f[9 + k])) builder.out.small = false;
-  }
-  const GpuTriangle* tris = (const GpuTriangle*)b.triangles;
-  size_t count = b.triangles_bytes / sizeof(GpuTriangle);
-  for (size_t i = 0; i < count; ++i) {
-    const GpuTriangle& t = tris[i];
-    TravTri& o = builder.out.tris[i];
-    for (int k = 0; k < 3; ++k) {
-      o.a[k] = t.a[k];
-      o.e1[k] = t.b[k] - t.a[k];  // tri_hit: e1 = tri.b.xyz - tri.a.xyz
-      o.e2[k] = t.c[k] - t.a[k];  // e2 = tri.c.xyz - tri.a.xyz
-    }
   }
   return std::move(builder.out);
 }

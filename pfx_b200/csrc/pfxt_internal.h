@@ -77,7 +77,9 @@ void set_error(const std::string& message);
 // Convert reference nodes into the B200 traversal layout (layout.cpp).
 struct TraversalLayout {
   std::vector<WideNode> wide;
-  std::vector<TravTri> tris;
+  // Per triangle slot the leaf that holds it, as wide node << 1 | child (REF_NONE:
+  // in no leaf); the device makes the triangles with it (k_lay_triangles).
+  std::vector<uint32_t> leaf_of;
   std::vector<InstRec> insts;
   uint32_t root = REF_NONE;  // wide node whose child 0 is the scene root
   bool small = false;        // every box coordinate 0 or within 2^-70..2^79 in magnitude (SceneView::small)

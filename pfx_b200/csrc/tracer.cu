@@ -1772,6 +1772,8 @@ void light_trig_init(pfxt_trace& t) {
   t.owned.push_back(d);
   t.shade.light_trig = static_cast<const float4*>(d);
   if (t.light_rows) {
+    // the rows' copy from pageable memory may still be under way, and t.stream does not wait for it
+    check(cudaStreamSynchronize(nullptr), "light-row trigonometry");
     k_light_trig<<<(t.light_rows + 127u) / 128u, 128, 0, t.stream>>>(t.shade, t.light_rows, static_cast<float4*>(d));
     k_pick_rows<<<(t.light_rows + 127u) / 128u, 128, 0, t.stream>>>(t.shade, t.light_rows,
                                                                     static_cast<PickRow*>(picks));

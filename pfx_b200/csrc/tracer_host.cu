@@ -44,14 +44,48 @@ T* dev_alloc(pfxt_trace& t, size_t count, const char* what) {
   return static_cast<T*>(dev_copy(t, nullptr, count * sizeof(T), what));
 }
 
-// The four-box nodes of `n` two-box nodes on the device.
-QuadNode* dev_quads(pfxt_trace& t, const WideNode* wide, size_t n) {
-  QuadNode* d = nullptr;
-  check(cudaMalloc(&d, std::max<size_t>(n, 1) * sizeof(QuadNode)), "nodes");
+// Device memory that is written by a kernel before it is read.
+template <typename T>
+T* dev_raw(pfxt_trace& t, size_t count, const char* what) {
+  T* d = nullptr;
+  check(cudaMalloc(&d, std::max<size_t>(count, 1) * sizeof(T)), what);
   t.owned.push_back(d);
-  check(launch_collapse(wide, (uint32_t)n, d, t.stream), "nodes");
-  check(cudaStreamSynchronize(t.stream), "nodes");
   return d;
+}
+
+void dev_free(pfxt_trace& t, void* p) {
+  auto it = std::find(t.owned.begin(), t.owned.end(), p);
+  if (it == t.owned.end()) return;
+  t.owned.erase(it);
+  cudaFree(p);
+}
+
+// The traversal buffers of a layout: uploaded, and what the device makes of them
+// and of the triangle records (`records`, on the device).
+struct Walkable {
+  WideNode* wide;
+  TravTri* tris;
+  InstRec* insts;
+  QuadNode* quad;
+};
+
+Walkable dev_walkable(pfxt_trace& t, const TraversalLayout& layout, const void* records) {
+  Walkable w;
+  w.wide = static_cast<WideNode*>(dev_copy(t, layout.wide.data(), layout.wide.size() * sizeof(WideNode), "nodes"));
+  w.insts =
+      static_cast<InstRec*>(dev_copy(t, layout.insts.data(), layout.insts.size() * sizeof(InstRec), "instances"));
+  void* leaf_of = dev_copy(t, layout.leaf_of.data(), layout.leaf_of.size() * sizeof(uint32_t), "triangles");
+  w.tris = dev_raw<TravTri>(t, layout.leaf_of.size(), "triangles");
+  w.quad = dev_raw<QuadNode>(t, layout.wide.size(), "nodes");
+  // a copy from pageable memory may still be under way, and t.stream does not wait for it
+  check(cudaStreamSynchronize(nullptr), "nodes");
+  check(launch_lay_triangles(static_cast<const GpuTriangle*>(records), static_cast<const uint32_t*>(leaf_of),
+                             (uint32_t)layout.leaf_of.size(), w.wide, w.tris, t.stream),
+        "triangles");
+  check(launch_collapse(w.wide, (uint32_t)layout.wide.size(), w.quad, t.stream), "nodes");
+  check(cudaStreamSynchronize(t.stream), "nodes");
+  dev_free(t, leaf_of);
+  return w;
 }
 
 bool finite3(const float* p) { return std::isfinite(p[0]) && std::isfinite(p[1]) && std::isfinite(p[2]); }
@@ -80,11 +114,12 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
 
   // ---- traversal layout
   TraversalLayout layout = make_layout(b);
-  t.d_wide = static_cast<WideNode*>(dev_copy(t, layout.wide.data(), layout.wide.size() * sizeof(WideNode), "nodes"));
-  t.d_tris = static_cast<TravTri*>(dev_copy(t, layout.tris.data(), layout.tris.size() * sizeof(TravTri), "triangles"));
-  t.d_insts =
-      static_cast<InstRec*>(dev_copy(t, layout.insts.data(), layout.insts.size() * sizeof(InstRec), "instances"));
-  t.d_quad = dev_quads(t, t.d_wide, layout.wide.size());
+  t.d_triangles = dev_copy(t, b.triangles, b.triangles_bytes, "triangle records");
+  const Walkable walkable = dev_walkable(t, layout, t.d_triangles);
+  t.d_wide = walkable.wide;
+  t.d_tris = walkable.tris;
+  t.d_insts = walkable.insts;
+  t.d_quad = walkable.quad;
   t.view.wide = t.d_wide;
   t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;
@@ -100,7 +135,6 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
   }
 
   // ---- shading buffers (reference layouts)
-  t.d_triangles = dev_copy(t, b.triangles, b.triangles_bytes, "triangle records");
   t.d_uv = dev_copy(t, b.uv, b.uv_bytes, "uv");
   t.d_materials = dev_copy(t, b.materials, b.materials_bytes, "materials");
   t.d_surfaces = dev_copy(t, b.surfaces, b.surfaces_bytes, "surfaces");
@@ -321,29 +355,22 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b) {
   check(cudaStreamSynchronize(t.stream), "move instances");
   // New traversal buffers first, so that a failed allocation leaves the trace as it was.
   size_t kept = t.owned.size();
-  void* fresh[4] = {nullptr, nullptr, nullptr, nullptr};
+  Walkable fresh;
   try {
-    fresh[0] = dev_copy(t, layout.wide.data(), layout.wide.size() * sizeof(WideNode), "nodes");
-    fresh[1] = dev_copy(t, layout.tris.data(), layout.tris.size() * sizeof(TravTri), "triangles");
-    fresh[2] = dev_copy(t, layout.insts.data(), layout.insts.size() * sizeof(InstRec), "instances");
-    fresh[3] = dev_quads(t, static_cast<const WideNode*>(fresh[0]), layout.wide.size());
+    void* records = dev_copy(t, b.triangles, b.triangles_bytes, "triangle records");
+    fresh = dev_walkable(t, layout, records);
+    dev_free(t, records);
   } catch (...) {
     for (size_t i = kept; i < t.owned.size(); ++i) cudaFree(t.owned[i]);
     t.owned.resize(kept);
     throw;
   }
   void* stale[4] = {t.d_wide, t.d_tris, t.d_insts, t.d_quad};
-  for (void* p : stale) {
-    auto it = std::find(t.owned.begin(), t.owned.end(), p);
-    if (it != t.owned.end()) {
-      t.owned.erase(it);
-      cudaFree(p);
-    }
-  }
-  t.d_wide = static_cast<WideNode*>(fresh[0]);
-  t.d_tris = static_cast<TravTri*>(fresh[1]);
-  t.d_insts = static_cast<InstRec*>(fresh[2]);
-  t.d_quad = static_cast<QuadNode*>(fresh[3]);
+  for (void* p : stale) dev_free(t, p);
+  t.d_wide = fresh.wide;
+  t.d_tris = fresh.tris;
+  t.d_insts = fresh.insts;
+  t.d_quad = fresh.quad;
   t.view.wide = t.d_wide;
   t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;

@@ -64,6 +64,19 @@ def test_small_trees(gpu, count, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("count", [127, 128, 129, 257])
+def test_the_last_triangles_of_a_block(gpu, count):
+    """The triangles are laid out by blocks of 128: rays at the last ones of a full and of a short block."""
+    rng = np.random.default_rng(count)
+    v = rng.uniform(-4, 4, (count, 1, 3)) + rng.uniform(-0.5, 0.5, (count, 3, 3))
+    scene = SceneDesc(synth.triangles(v.astype(F32)), synth.material(), synth.look_at((0, 0, 10), (0, 0, 0), 45, 1.0))
+    aim = np.repeat(v.mean(1), 4, 0).astype(F32)
+    o = rng.uniform(-6, 6, aim.shape).astype(F32)
+    hits = compare(Trace(scene, Settings(), 8, 8), oracle.scene_buffers(scene, Settings()), make_rays(o, aim - o, 1e20))
+    assert hits == len(o)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["doubled", "needles", "stacked", "grid", "mixed"])
 def test_ties_and_slivers(gpu, kind):
     """Where the order of the walk could show: the same triangles twice, needles
