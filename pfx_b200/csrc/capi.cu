@@ -453,6 +453,17 @@ int pfxt_debug_select_nth(const float* keys, uint32_t n, uint32_t index, int32_t
   });
 }
 
+/* What the traversal layout of a scene's buffers says of them: whether the
+ * four-box walk takes their rays, and the entries its stack can come to hold. */
+int pfxt_debug_layout(const pfxt_buffers* b, uint32_t* small, uint32_t* stack_need) {
+  return guarded([&]() {
+    if (!b || !small || !stack_need) throw Invalid("null argument");
+    const TraversalLayout layout = make_layout(*b);
+    *small = layout.small ? 1u : 0u;
+    *stack_need = layout.stack_need;
+  });
+}
+
 /* Large triangle BVHs on the GPU (1, the default, when a device is present) or
  * always on the host (0); returns the previous setting.  The bytes are the same. */
 int pfxt_debug_gpu_bvh(int32_t on) { return set_gpu_bvh(on); }

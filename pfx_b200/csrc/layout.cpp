@@ -52,18 +52,19 @@ struct Builder {
   uint32_t base = 0;
   std::unordered_map<uint32_t, uint32_t> base_of;
   bool unboxed = false;
-  // Entries the four-box walk's stack needs (the buffers' own max_depth is the
-  // caller's word, and the two-box walk's): below the child laid out last as one
-  // entry, and below its own two children when it is an inner node; below each
-  // pseudo-parent's root as a node of its own.
+  // Entries the four-box walk's stack can come to hold, whichever of a node's
+  // children it enters first (any hits go to the nearest one; the buffers' own
+  // max_depth is the caller's word, and the two-box walk's): below the child
+  // laid out last as one entry, and below its own two children when it is an
+  // inner node; below each pseudo-parent's root as a node of its own.
   struct Need {
     uint32_t whole = 0, child[2] = {0, 0};
     bool inner = false;
   } need;
   std::unordered_map<uint32_t, uint32_t> need_of;
 
-  // Of a node whose children need l and r: inside entry i of its four, the
-  // entries after i wait.
+  // Of a node whose children need l and r: inside any entry of its up to four,
+  // all the others may wait.
   static uint32_t quad_need(const Need& l, const Need& r) {
     uint32_t list[4], n = 0, most = 0;
     for (const Need* c : {&l, &r}) {
@@ -74,8 +75,8 @@ struct Builder {
         list[n++] = c->whole;
       }
     }
-    for (uint32_t i = 0; i < n; ++i) most = std::max(most, n - 1u - i + list[i]);
-    return most;
+    for (uint32_t i = 0; i < n; ++i) most = std::max(most, list[i]);
+    return n - 1u + most;
   }
 
   // The leaf `at` (wide node << 1 | child, whose box the wide node has already).
@@ -214,14 +215,14 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
     // the top level itself: world leaves (base 0) must stay inside the triangles
     if (builder.reach_of[builder.out.root] > builder.tri_count)
       throw Invalid("a BVH leaf reaches past the triangles");
-    if (builder.need_of[builder.out.root] > QUAD_STACK) builder.unboxed = true;
+    builder.out.stack_need = builder.need_of[builder.out.root];
   }
   // The box test needs no range check on its quotients when every box
   // coordinate is 0 or of magnitude in [2^-70, 2^79] (traverse.cuh,
   // BOUNDED_TINY and BOUNDED_COORD); NaN coordinates fail this too.  The
   // four-box walk also picks the planes that a ray enters through by its
   // direction's signs, which asks for lo <= hi, and leaves whose triangles
-  // know their box, and a stack that fits QUAD_STACK entries.
+  // know their box.
   builder.out.small = !builder.unboxed;
   for (const WideNode& w : builder.out.wide) {
     const float* f = &w.b0[0];

@@ -82,6 +82,7 @@ struct TraversalLayout {
   std::vector<uint32_t> leaf_of;
   std::vector<InstRec> insts;
   uint32_t root = REF_NONE;  // wide node whose child 0 is the scene root
+  uint32_t stack_need = 0;   // entries the four-box walk's stack can come to hold, in any order
   bool small = false;        // every box coordinate 0 or within 2^-70..2^79 in magnitude (SceneView::small)
 };
 TraversalLayout make_layout(const pfxt_buffers& buffers);

@@ -132,9 +132,9 @@ static_assert(sizeof(InstRec) == 96, "InstRec");
 constexpr uint32_t REF_STACK = 64u;
 // Stack entries of the four-box walk.  It waits on up to three siblings a node
 // where the reference waits on one per level; layout.cpp works out what a
-// scene needs, and one that needs more takes the two-box walk.  (The 1.19 M
-// triangle room needs under 40; 128 entries made the local memory of every
-// resident thread 1 KB.)
+// scene's rays can come to hold, and where that is more the walk checks for room
+// and hands over a ray that has none.  (The 1.19 M triangle room needs 39; 128
+// entries made the local memory of every resident thread 1 KB.)
 constexpr uint32_t QUAD_STACK = 64u;
 
 }  // namespace pfxt

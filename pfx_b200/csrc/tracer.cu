@@ -483,8 +483,8 @@ __global__ void k_rewind(const __grid_constant__ Pass P, uint32_t cur) {
 // THREADS per block is a launch choice of the autotuner: the walk is per lane
 // and the refill per warp, so the block size changes only the residency.
 // SHORT entries of each lane's traversal stack live in shared memory (a tuning
-// choice: 0 or 8), the rest in local memory.
-template <bool ANY, int THREADS, int SHORT>
+// choice: 0 or 8), the rest in local memory.  GUARD: QuadWalker's, for deep scenes.
+template <bool ANY, int THREADS, int SHORT, bool GUARD = false>
 __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_trace_queue(const __grid_constant__ Pass P,
                                                                                        uint32_t which) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
     st.sh_near = short_near + threadIdx.x;
     st.lanes = THREADS;
   }
-  QuadWalker<ANY> w;
+  QuadWalker<ANY, GUARD> w;
   w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0, item = 0;
@@ -1559,10 +1559,14 @@ void launch_trace_queue_short(int sel, const Pass& P, uint32_t which, cudaStream
 
 template <bool ANY>
 void launch_trace_queue(int sel, uint32_t short_stack, const Pass& P, uint32_t which, cudaStream_t st) {
-  if (short_stack > 0u)
+  if (P.s.deep != 0u) {  // rare: one launch shape, whatever the tuning
+    static const int blocks = grid_for((const void*)k_trace_queue<ANY, 128, 0, true>, 128);
+    k_trace_queue<ANY, 128, 0, true><<<blocks, 128, 0, st>>>(P, which);
+  } else if (short_stack > 0u) {
     launch_trace_queue_short<ANY, 8>(sel, P, which, st);
-  else
+  } else {
     launch_trace_queue_short<ANY, 0>(sel, P, which, st);
+  }
   k_trace_queue_retry<ANY><<<grids().retry, 128, 0, st>>>(P);
 }
 

@@ -38,13 +38,13 @@ constexpr uint32_t RETRY = QuadWalker<true>::RETRY;
 
 // MODE 0: closest hit -> pfxt_hit; MODE 1: any hit -> u32 flag.  Rays that the
 // four-box walk cannot take are marked RETRY for k_trace_retry.
-template <int MODE>
+template <int MODE, bool GUARD = false>
 __global__ void __launch_bounds__(kThreads, TRACE_WARPS_PER_SM * 32 / kThreads) k_trace(SceneView s, const pfxt_ray* __restrict__ rays, uint32_t n,
                                                     void* __restrict__ out, uint32_t* __restrict__ counter, uint32_t lanes) {
   constexpr bool ANY = MODE == 1;
   constexpr unsigned FULL = 0xffffffffu;
   QuadStack st;
-  QuadWalker<ANY> w;
+  QuadWalker<ANY, GUARD> w;
   w.idle();
   const int lane = threadIdx.x & 31;
   uint32_t idx = 0;
@@ -217,7 +217,7 @@ constexpr int kMaxDevices = 64;
 // Blocks of a persistent launch on the current device (SM count x resident
 // blocks), computed once per device.  Threads that race on a device's first
 // launch compute the same number, so the relaxed store is enough.
-template <int MODE>
+template <int MODE, bool GUARD = false>
 int persistent_blocks() {
   static std::atomic<int> cached[kMaxDevices];
   int dev = 0;
@@ -227,23 +227,23 @@ int persistent_blocks() {
   if (blocks == 0) {
     int sms = 0, per = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<MODE>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<MODE, GUARD>, kThreads, 0);
     blocks = (sms > 0 ? sms : 1) * (per > 0 ? per : 1);
     if (slot) slot->store(blocks, std::memory_order_relaxed);
   }
   return blocks;
 }
 
-template <int MODE>
+template <int MODE, bool GUARD>
 cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* out, uint32_t* counter,
                    cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
-  const uint32_t most = (uint32_t)persistent_blocks<MODE>();
+  const uint32_t most = (uint32_t)persistent_blocks<MODE, GUARD>();
   const uint32_t lanes = lanes_per_warp(n, most * (kThreads / 32));
   const uint32_t blocks = std::min(most, (n + lanes * (kThreads / 32) - 1) / (lanes * (kThreads / 32)));
-  k_trace<MODE><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter, lanes);
+  k_trace<MODE, GUARD><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter, lanes);
   k_trace_retry<MODE><<<std::min(most, (n + kThreads - 1) / kThreads), kThreads, 0, stream>>>(s, rays, n, out);
   return cudaGetLastError();
 }
@@ -252,12 +252,14 @@ cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* o
 
 cudaError_t launch_closest(const SceneView& s, const pfxt_ray* rays, uint32_t n, pfxt_hit* hits, uint32_t* counter,
                            cudaStream_t stream) {
-  return launch<0>(s, rays, n, hits, counter, stream);
+  return s.deep ? launch<0, true>(s, rays, n, hits, counter, stream)
+                : launch<0, false>(s, rays, n, hits, counter, stream);
 }
 
 cudaError_t launch_any(const SceneView& s, const pfxt_ray* rays, uint32_t n, uint32_t* blocked, uint32_t* counter,
                        cudaStream_t stream) {
-  return launch<1>(s, rays, n, blocked, counter, stream);
+  return s.deep ? launch<1, true>(s, rays, n, blocked, counter, stream)
+                : launch<1, false>(s, rays, n, blocked, counter, stream);
 }
 
 cudaError_t launch_counts(const SceneView& s, const pfxt_ray* rays, uint32_t n, bool any, uint2* counts,
@@ -286,8 +288,10 @@ cudaError_t launch_lay_triangles(const GpuTriangle* records, const uint32_t* lea
 
 cudaError_t prepare_any_queries() {
   persistent_blocks<1>();
+  persistent_blocks<1, true>();
   cudaFuncAttributes attr;
   cudaError_t e = cudaFuncGetAttributes(&attr, k_trace<1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, k_trace<1, true>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, k_trace_retry<1>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, k_pack);
   return e;
