@@ -222,7 +222,9 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
   // BOUNDED_TINY and BOUNDED_COORD); NaN coordinates fail this too.  The
   // four-box walk also picks the planes that a ray enters through by its
   // direction's signs, which asks for lo <= hi, and leaves whose triangles
-  // know their box.
+  // know their box.  And it
+  // passes over the boxes between a leaf and the root, which a leaf that passes
+  // implies only where every box holds its children's.
   builder.out.small = !builder.unboxed;
   for (const WideNode& w : builder.out.wide) {
     const float* f = &w.b0[0];
@@ -232,6 +234,14 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
     }
     for (int k = 0; k < 3; ++k)
       if (!(f[k] <= f[3 + k]) || !(f[6 + k] <= f[9 + k])) builder.out.small = false;
+    for (int c = 0; c < 2; ++c) {
+      if (w.child[c] & REF_LEAF) continue;  // a leaf, an instance or none
+      const WideNode& below = builder.out.wide[w.child[c]];
+      const float* b = &below.b0[0];
+      for (int k = 0; k < 3; ++k)
+        for (int j = 0; j < (below.child[1] == REF_NONE ? 1 : 2); ++j)
+          if (!(b[6 * j + k] >= f[6 * c + k]) || !(b[6 * j + 3 + k] <= f[6 * c + 3 + k])) builder.out.small = false;
+    }
   }
   return std::move(builder.out);
 }

@@ -1504,7 +1504,7 @@ struct Grids {
   // [threads choice (64, 128, 256)][shared-memory stack entries (0, 8)]
   int trace_closest[3][2] = {}, trace_any[3][2] = {}, shade = 0, shade_inline = 0, flat = 0;
   int shade_hit = 0, shade_lights = 0, shade_lights_inline = 0, shade_bsdf = 0;
-  int retry = 0;  // blocks of the retry walks: one per SM (their work is rare)
+  int retry = 0;  // blocks of the retry walks: one per SM (their work is rare, but in scenes that are not `small`)
   int tree_pick = 0, slot[5] = {};  // the light slots, one kind per launch
 };
 Grids& grids() {
@@ -1567,7 +1567,7 @@ void launch_trace_queue(int sel, uint32_t short_stack, const Pass& P, uint32_t w
   } else {
     launch_trace_queue_short<ANY, 0>(sel, P, which, st);
   }
-  k_trace_queue_retry<ANY><<<grids().retry, 128, 0, st>>>(P);
+  k_trace_queue_retry<ANY><<<grids().retry * (P.s.small != 0u ? 1 : 8), 128, 0, st>>>(P);
 }
 
 int thread_select(uint32_t threads) { return threads == 64u ? 0 : (threads == 256u ? 2 : 1); }

@@ -52,7 +52,7 @@ struct SceneView {
   const InstRec* __restrict__ insts;
   uint32_t root;
   uint32_t small;  // 1 when every box coordinate is 0 or in [BOUNDED_TINY, BOUNDED_COORD] in magnitude,
-                   // lo <= hi, and every leaf's triangles hold its box
+                   // lo <= hi, every box holds its children's, and every leaf's triangles hold its box
   uint32_t deep;   // 1 when a ray may come to hold more than QUAD_STACK entries: QuadWalker's GUARD
 };
 
