@@ -424,8 +424,8 @@ int pfxt_debug_rays(pfxt_trace* t, uint64_t* out) {
  * the stream the passes run on. */
 void* pfxt_debug_stream(pfxt_trace* t) { return t ? (void*)t->stream : nullptr; }
 
-/* Turn the per-bounce material sort of the shade queue on (1, the default) or
- * off (0); the image does not change, only the time. */
+/* Turn the per-bounce material sort of the shade queue on (1) or off (0, the
+ * default); the image does not change, only the time. */
 int pfxt_debug_sort(pfxt_trace* t, uint32_t on) {
   return guarded([&]() {
     if (!t) throw Invalid("null argument");

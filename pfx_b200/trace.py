@@ -465,7 +465,7 @@ class Trace:
                 "shadow_queue": bool(k.shadow_queue), "short_stack": int(k.short_stack),
                 "from_cache": bool(k.from_cache), "slot_kernels": bool(k.slot_kernels)}
 
-    def set_tuning(self, trace_threads: int = 128, sort_shading: bool = True, graphs: bool = True,
+    def set_tuning(self, trace_threads: int = 128, sort_shading: bool = False, graphs: bool = True,
                    split_shade: bool = True, sort_rays: bool = False, shadow_queue: bool = True,
                    short_stack: int = 0, slot_kernels: bool = True) -> None:
         k = abi.Tuning(trace_threads, int(sort_shading), int(graphs), int(split_shade), int(sort_rays), 0.0,
