@@ -1638,6 +1638,7 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
     }
     buffer = nullptr;
     held = 0;
+    if (wide) t.wide_capacity = 0u;
     const cudaError_t e = cudaMalloc(&buffer, need);
     if (e != cudaSuccess) buffer = nullptr;
     if (wide && e == cudaErrorMemoryAllocation) {  // another program took the memory meanwhile
@@ -1646,6 +1647,7 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
     }
     check(e, "wavefront path state");
     held = need;
+    if (wide) t.wide_capacity = capacity;
   }
   char* b = static_cast<char*>(buffer);
   Wave& w = *reinterpret_cast<Wave*>(&t.wave_layout);
@@ -1820,12 +1822,22 @@ void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed, uint32_t live) {
   bool deferred = slots <= CAP_MAX && t.shadow_queue;
   // The cache's queries and training paths are counted per sample: one at a time.
   uint32_t shift = t.cache ? 0u : wave_shift(live, count);
-  uint32_t capacity = shift > 0u ? std::max(pixels, WAVE_PATHS) : pixels;
-  if (shift > 0u && !ensure_wave(t, capacity, cap, true)) {
-    shift = 0u;
-    capacity = pixels;
+  bool wide = false;
+  if (shift > 0u) {
+    // buffers that one sample of the film does not need: as many paths as this
+    // call takes, in powers of two, so that a growing call seldom finds them short
+    const uint32_t paths = live << shift;
+    if (paths > std::max(pixels, t.wide_capacity)) {
+      uint32_t most = 1u;
+      while (most < paths) most <<= 1;
+      ensure_wave(t, most, cap, true);  // without room for them, the waves fit what there is
+    }
+    const uint32_t hold = std::max(pixels, t.wide_capacity);
+    while ((uint64_t)live << shift > hold) --shift;
+    wide = shift > 0u && t.wide_capacity > 0u;
   }
-  if (shift == 0u) ensure_wave(t, capacity, cap, false);
+  const uint32_t capacity = wide ? t.wide_capacity : pixels;
+  ensure_wave(t, capacity, cap, wide);
   Pass P;
   memset(&P, 0, sizeof(P));
   P.shift = shift;

@@ -119,6 +119,7 @@ struct pfxt_trace {
   size_t wave_bytes = 0;
   void* d_wide_wave = nullptr;  // of waves of several samples a pixel
   size_t wide_wave_bytes = 0;
+  uint32_t wide_capacity = 0;  // paths they hold: 0, or more than the film's pixels
   alignas(16) unsigned char wave_layout[256];  // pointers into one of them (tracer.cu)
   uint32_t light_rows = 0;                     // rows of the light buffer (lights + tree)
   uint32_t* wave_counters = nullptr;           // queue counters and ray totals
