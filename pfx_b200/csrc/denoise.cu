@@ -568,11 +568,12 @@ __global__ void __launch_bounds__(ws_threads<S>(), 1) k_conv_ws(const __grid_con
   const uint32_t chunks = (a.c0 + a.c1) >> 4, chunks0 = a.c0 >> 4;
   const uint32_t wbytes = 9u * 2u * a.n * 16u;
   // Every CTA of this grid is resident (one per SM at most), so the next layer's
-  // may come in where SMs are free; nothing is read or written here before the
-  // layers before this one are done (the other warps' work follows from the copies).
+  // may come in where SMs are free.  Every thread waits for the layers before this
+  // one: the copies may not start earlier, and the polls of the other warps are to
+  // count this layer's time alone (wait_limit).
+  if (tid == 0) umma::launch_dependents();
+  umma::wait_prerequisites();
   if (tid == 0) {  // the copies
-    umma::launch_dependents();
-    umma::wait_prerequisites();
     uint32_t c = 0, u = 0;  // chunks, raw copies
     for (uint32_t t = blockIdx.x; t < tiles && !*abort_flag; t += gridDim.x) {
       const int x0 = (int)((t % gx) * CONV_PIX), y0 = (int)((t / gx) * ROWS);
