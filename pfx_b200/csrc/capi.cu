@@ -641,6 +641,7 @@ void restore_checkpoint(pfxt_trace& t, const Checkpoint& c) {
   float4* films[3] = {t.d_color, t.d_albedo, t.d_normal};
   for (int k = 0; k < 3; ++k)
     check(cudaMemcpy(films[k], c.films[k], pixels * CKPT_TEXEL, cudaMemcpyHostToDevice), "restore");
+  check(cudaStreamSynchronize(nullptr), "restore");  // t.stream does not wait for the default stream
   t.samples = c.samples;
 }
 
@@ -679,6 +680,7 @@ int pfxt_sample_adaptive_kept(pfxt_trace* t, const pfxt_adaptive* a, uint32_t se
       restore_checkpoint(*t, c);
       const uint64_t pixels = (uint64_t)t->width * t->height;
       check(cudaMemcpy(t->d_snaps, c.snaps, pixels * CKPT_SNAP, cudaMemcpyHostToDevice), "restore");
+      check(cudaStreamSynchronize(nullptr), "restore");
       for (uint32_t r = 0; r < c.rounds; ++r) {
         pfxt_round round{0u, 0u, 0u};
         memcpy(&round.samples, c.round_bytes + 12 * r, 4);

@@ -1607,7 +1607,7 @@ bool ensure_wave(pfxt_trace& t, uint32_t capacity, uint32_t cap, bool wide) {
     void* d = nullptr;
     check(cudaMalloc(&d, 128), "counters");
     t.owned.push_back(d);
-    check(cudaMemset(d, 0, 128), "counters");
+    check(cudaMemsetAsync(d, 0, 128, t.stream), "counters");  // the passes' own stream
     t.wave_counters = static_cast<uint32_t*>(d);
   }
   void*& buffer = wide ? t.d_wide_wave : t.d_wave;

@@ -274,6 +274,8 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
   t.tune_key = tune_key_of(b, sp, width, height);
 
   light_trig_init(t);
+  // t.stream does not wait for the copies and memsets that the default stream still has under way
+  check(cudaStreamSynchronize(nullptr), "scene upload");
 }
 
 void trace_release(pfxt_trace& t) {
@@ -383,6 +385,7 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b) {
   check(cudaMemcpy(t.d_emitters, b.emitters, b.emitters_bytes, cudaMemcpyHostToDevice), "emitters");
   if (b.emitter_cdf_bytes)
     check(cudaMemcpy(t.d_emitter_cdf, b.emitter_cdf, b.emitter_cdf_bytes, cudaMemcpyHostToDevice), "emitter cdf");
+  check(cudaStreamSynchronize(nullptr), "scene upload");  // as at creation
   const GpuNode* root = static_cast<const GpuNode*>(b.nodes);
   for (int k = 0; k < 3; ++k) {
     t.bounds_lo[k] = root->lo[k];
