@@ -52,6 +52,7 @@ struct Builder {
   uint32_t base = 0;
   std::unordered_map<uint32_t, uint32_t> base_of;
   bool unboxed = false;
+  bool uncontained = false;  // a box does not hold a child's
   // Entries the four-box walk's stack can come to hold, whichever of a node's
   // children it enters first (any hits go to the nearest one; the buffers' own
   // max_depth is the caller's word, and the two-box walk's): below the child
@@ -184,6 +185,9 @@ struct Builder {
     WideNode node{};
     set_box(node, 0, nodes[left]);
     set_box(node, 1, nodes[right]);
+    for (const GpuNode* c : {&nodes[left], &nodes[right]})
+      for (int k = 0; k < 3; ++k)
+        if (!(c->lo[k] >= n.lo[k]) || !(c->hi[k] <= n.hi[k])) uncontained = true;
     out.wide[w] = node;
     node.child[0] = child_ref(left, w << 1);
     const Need l = need;
@@ -225,7 +229,7 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
   // know their box.  And it
   // passes over the boxes between a leaf and the root, which a leaf that passes
   // implies only where every box holds its children's.
-  builder.out.small = !builder.unboxed;
+  builder.out.small = !builder.unboxed && !builder.uncontained;
   for (const WideNode& w : builder.out.wide) {
     const float* f = &w.b0[0];
     for (int k = 0; k < 12; ++k) {
@@ -234,14 +238,6 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
     }
     for (int k = 0; k < 3; ++k)
       if (!(f[k] <= f[3 + k]) || !(f[6 + k] <= f[9 + k])) builder.out.small = false;
-    for (int c = 0; c < 2; ++c) {
-      if (w.child[c] & REF_LEAF) continue;  // a leaf, an instance or none
-      const WideNode& below = builder.out.wide[w.child[c]];
-      const float* b = &below.b0[0];
-      for (int k = 0; k < 3; ++k)
-        for (int j = 0; j < (below.child[1] == REF_NONE ? 1 : 2); ++j)
-          if (!(b[6 * j + k] >= f[6 * c + k]) || !(b[6 * j + 3 + k] <= f[6 * c + 3 + k])) builder.out.small = false;
-    }
   }
   return std::move(builder.out);
 }
