@@ -746,7 +746,7 @@ int pfxt_finish_tops(pfxt_trace* t, const pfxt_buffers* b) {
     if (b->max_depth > REF_STACK) throw Invalid("the BVH needs more than the 64-entry traversal stack");
     if (b->nodes_bytes % sizeof(GpuNode) || b->triangles_bytes % sizeof(GpuTriangle))
       throw Invalid("scene buffers have invalid sizes");
-    trace_move_scene(*t, *b);
+    trace_move_scene(*t, *b, false);
     if (t->cache) bind_cache_bounds(*t, *t->cache);
   });
 }
@@ -760,7 +760,7 @@ int pfxt_set_instance_transforms(pfxt_trace* t, pfxt_scene_blobs* h, const float
     if (h->blobs->max_depth > REF_STACK) throw Invalid("the BVH needs more than the 64-entry traversal stack");
     pfxt_buffers b;
     if (pfxt_scene_buffers(h, &b) != PFXT_OK) throw Invalid(pfxt_last_error());
-    trace_move_scene(*t, b);
+    trace_move_scene(*t, b, true);
     if (t->cache) bind_cache_bounds(*t, *t->cache);
     if (moved) *moved = 1u;
   });
