@@ -226,7 +226,8 @@ constexpr uint32_t A_PLANE = PATCH_W * 16u;          // bytes of one (row, group
 // (384 of 512 TMEM columns): 6.62 ms, the same image bit for bit.
 // With the MMAs over up to three output rows 6.73 ms where the form before took
 // 7.22 (later boxes), with two epilogue warps a quarter 5.70, with tiles of 126
-// pixels 4.87, with each layer's set-up beside the layer before it 4.82.
+// pixels 4.87, with each layer's set-up beside the layer before it 4.82 (the
+// same films every time; 5.57 over films that change).
 template <uint32_t ROWS_, uint32_t NMAX_, uint32_t STAGES_, uint32_t CTAS_, bool EXPAND_ = false,
           uint32_t RAWS_ = 1>
 struct ConvShape {

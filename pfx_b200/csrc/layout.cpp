@@ -224,11 +224,9 @@ TraversalLayout make_layout(const pfxt_buffers& b) {
   // The box test needs no range check on its quotients when every box
   // coordinate is 0 or of magnitude in [2^-70, 2^79] (traverse.cuh,
   // BOUNDED_TINY and BOUNDED_COORD); NaN coordinates fail this too.  The
-  // four-box walk also picks the planes that a ray enters through by its
-  // direction's signs, which asks for lo <= hi, and leaves whose triangles
-  // know their box.  And it
-  // passes over the boxes between a leaf and the root, which a leaf that passes
-  // implies only where every box holds its children's.
+  // four-box walk also passes over the boxes between a leaf and the root, which a
+  // leaf that passes implies only where lo <= hi and every box holds its
+  // children's, and needs leaves whose triangles know their box.
   builder.out.small = !builder.unboxed && !builder.uncontained;
   for (const WideNode& w : builder.out.wide) {
     const float* f = &w.b0[0];

@@ -97,7 +97,8 @@ static_assert(sizeof(WideNode) == 64, "WideNode");
 // Four-box node of the closest- and any-hit walks: the grandchildren of an
 // inner node (or a child itself where it is a leaf), in the reference's
 // left-first order: one 32-byte sector of planes an axis and one with the
-// references.  Unused children hold the empty box (+inf, -inf).
+// references.  Unused children come last, with planes at +inf and -inf (which the
+// walk's test does not fail: QuadWalker::open).
 struct alignas(128) QuadNode {
   struct {
     float lo[4], hi[4];
@@ -108,7 +109,7 @@ struct alignas(128) QuadNode {
 static_assert(sizeof(QuadNode) == 128, "QuadNode");
 
 // A triangle (vertex a, the two edges) and the exact box of the leaf that
-// holds it; the first three 16-byte words are all that the triangle test reads.
+// holds it; the first 36 bytes are all that the triangle test reads.
 struct alignas(64) TravTri {
   float a[3], e1[3], e2[3];  // a, b - a, c - a
   float lo[3], hi[3];        // the leaf's box

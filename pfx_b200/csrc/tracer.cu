@@ -151,7 +151,6 @@ struct Pass {
   uint32_t shift;      // log2 of the samples of a pixel in the wave
   uint32_t capacity;   // paths the wave's buffers hold
   uint32_t bounce;
-  uint32_t cap;        // shadow slots per path
   uint32_t deferred;   // 1: light-slot shadow rays go through the shadow queue
   uint32_t light_rows;
   uint32_t slots;      // 2 + light_slots()
@@ -1155,8 +1154,8 @@ __global__ void __launch_bounds__(kThreads, SHADE_LIGHTS_MIN_BLOCKS) k_shade_lig
 // keeps the union of every kind's state in local memory.  The values are the
 // same: a path's draws come in the same order (slot k's after slot k-1's; the
 // pcg state travels in thr.w between launches), and the k-th live slot of a
-// path writes shadow entry i * cap + pending, the pending count travelling in
-// the flag word.  The tree's slot is two launches: the descent (k_tree_pick,
+// path writes shadow entry pending * capacity + i, the pending count travelling
+// in the flag word.  The tree's slot is two launches: the descent (k_tree_pick,
 // one (row, pmf) per path), then its light's candidate and the BSDF.
 constexpr int SLOT_SUN = 0, SLOT_SKY = 1, SLOT_EMITTER = 2, SLOT_LOOPED = 3, SLOT_TREE = 4;
 
@@ -1851,7 +1850,6 @@ void trace_sample(pfxt_trace& t, uint32_t count, uint32_t seed, uint32_t live) {
   P.v = t.shade;
   P.s = t.view;
   P.w = *reinterpret_cast<Wave*>(&t.wave_layout);
-  P.cap = cap;
   P.deferred = deferred ? 1u : 0u;
   P.light_rows = t.light_rows;
   P.slots = slots;

@@ -129,7 +129,8 @@ struct pfxt_trace {
   // 4K pass); the split kernels lose more from gathering paths out of order:
   // sorted and unsorted, 1280 x 720 at 16 samples 90.0 and 77.9 ms, the 4K
   // pass 81.7 and 70.7, a 320 x 180 preview 1.52 and 1.40, 512 x 512 at 16
-  // samples 4.05 and 3.87, a cached 1080p pass 9.81 and 9.51.
+  // samples 4.05 and 3.87, a cached 1080p pass 9.81 and 9.51.  Not everywhere:
+  // the autotuner takes it for the cached 4K pass.
   bool sort_shading = false;
   uint32_t trace_threads = 128;                // threads per block of the traversal kernels (64, 128, 256)
   bool split_shade = true;                     // shade in three kernels (hit, lights, BSDF) or one

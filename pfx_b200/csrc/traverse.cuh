@@ -190,8 +190,8 @@ __device__ __forceinline__ bool box_geometry_bounded(float lx, float ly, float l
 }
 
 // Two fp32 lanes in one 64-bit register and the sm_100 paired instructions on
-// them: each lane is one IEEE round-to-nearest add, multiply or fused
-// multiply-add, the same operation as the scalar instruction, two per issue.
+// them: each lane is one IEEE round-to-nearest subtraction or multiplication,
+// the same operation as the scalar instruction, two per issue.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pair(float lo, float hi) {
   f32x2 r;
@@ -209,11 +209,6 @@ __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
 
@@ -530,9 +525,9 @@ struct Walker {
 // The loose test.  A plane's quotient is x * r with x = lo - o rounded as the
 // reference rounds it and r within an ulp of 1/d: within 2^-21 of the
 // reference's quotient x / d in relative terms for a bounded ray (no
-// underflow), and the planes a ray enters and leaves through follow from the
-// signs of d (lo <= hi).  Entry <= exit and entry <= hit.t are compared with
-// the right side scaled by 1 + 2^-18, so a box that passes exactly passes here.
+// underflow); entry and exit are their minima and maxima as the reference takes
+// them.  Entry <= exit and entry <= hit.t are compared with the right side
+// scaled by 1 + 2^-18, so a box that passes exactly passes here.
 //
 // The exact test (box_exact) runs where it decides: before the first triangle
 // of a leaf is accepted, against the hit distance from before that leaf, and
@@ -581,9 +576,8 @@ constexpr int HOLDERS = 16;
 template <bool ANY, bool GUARD = false>
 struct QuadWalker {
   // the ray of the current space: origins and approximate reciprocals in both
-  // lanes of a pair (a node's planes come two children to a pair), the
-  // direction, and per axis the byte offset in a node of the planes it enters
-  // through
+  // lanes of a pair (a node's planes come two children to a pair), and the
+  // direction
   f32x2 ox, oy, oz, rx, ry, rz;
   v3 d;
   uint32_t inst;  // the instance the walk is in, REF_NONE in world space
@@ -682,7 +676,9 @@ struct QuadWalker {
 
   // Opens the inner node at hand: tests its four children loosely.  Closest hit:
   // the first that passes is next, the others are pushed last first; any hit:
-  // the nearest is next.
+  // the nearest is next.  An unused child passes too (its planes are both
+  // infinite), but unused children are last, so they are looked at while `next`
+  // is still REF_NONE, and leave it so: nothing is pushed for them.
   template <class Stack>
   __device__ __forceinline__ void open(const SceneView& s, Stack& st) {
     if (GUARD && top > Stack::CAPACITY - 3) {  // three children may wait
