@@ -1558,7 +1558,7 @@ void launch_trace_queue_short(int sel, const Pass& P, uint32_t which, cudaStream
 
 template <bool ANY>
 void launch_trace_queue(int sel, uint32_t short_stack, const Pass& P, uint32_t which, cudaStream_t st) {
-  if (P.s.deep != 0u) {  // rare: one launch shape, whatever the tuning
+  if (P.s.small == 2u) {  // rare: one launch shape, whatever the tuning
     static const int blocks = grid_for((const void*)k_trace_queue<ANY, 128, 0, true>, 128);
     k_trace_queue<ANY, 128, 0, true><<<blocks, 128, 0, st>>>(P, which);
   } else if (short_stack > 0u) {

@@ -126,8 +126,7 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
   t.view.tris = t.d_tris;
   t.view.insts = t.d_insts;
   t.view.root = layout.root;
-  t.view.small = layout.small ? 1u : 0u;
-  t.view.deep = layout.stack_need > QUAD_STACK ? 1u : 0u;
+  t.view.small = layout.small ? (layout.stack_need > QUAD_STACK ? 2u : 1u) : 0u;
   if (b.nodes_bytes >= sizeof(GpuNode)) {
     const GpuNode* root = static_cast<const GpuNode*>(b.nodes);
     for (int k = 0; k < 3; ++k) {
@@ -387,8 +386,7 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b, bool own) {
   t.view.tris = t.d_tris;
   t.view.insts = t.d_insts;
   t.view.root = layout.root;
-  t.view.small = layout.small ? 1u : 0u;
-  t.view.deep = layout.stack_need > QUAD_STACK ? 1u : 0u;
+  t.view.small = layout.small ? (layout.stack_need > QUAD_STACK ? 2u : 1u) : 0u;
   check(cudaMemcpy(t.d_surfaces, b.surfaces, b.surfaces_bytes, cudaMemcpyHostToDevice), "surfaces");
   check(cudaMemcpy(t.d_emitters, b.emitters, b.emitters_bytes, cudaMemcpyHostToDevice), "emitters");
   if (b.emitter_cdf_bytes)

@@ -252,14 +252,14 @@ cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* o
 
 cudaError_t launch_closest(const SceneView& s, const pfxt_ray* rays, uint32_t n, pfxt_hit* hits, uint32_t* counter,
                            cudaStream_t stream) {
-  return s.deep ? launch<0, true>(s, rays, n, hits, counter, stream)
-                : launch<0, false>(s, rays, n, hits, counter, stream);
+  return s.small == 2u ? launch<0, true>(s, rays, n, hits, counter, stream)
+                       : launch<0, false>(s, rays, n, hits, counter, stream);
 }
 
 cudaError_t launch_any(const SceneView& s, const pfxt_ray* rays, uint32_t n, uint32_t* blocked, uint32_t* counter,
                        cudaStream_t stream) {
-  return s.deep ? launch<1, true>(s, rays, n, blocked, counter, stream)
-                : launch<1, false>(s, rays, n, blocked, counter, stream);
+  return s.small == 2u ? launch<1, true>(s, rays, n, blocked, counter, stream)
+                       : launch<1, false>(s, rays, n, blocked, counter, stream);
 }
 
 cudaError_t launch_counts(const SceneView& s, const pfxt_ray* rays, uint32_t n, bool any, uint2* counts,

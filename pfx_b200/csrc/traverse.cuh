@@ -53,7 +53,7 @@ struct SceneView {
   uint32_t root;
   uint32_t small;  // 1 when every box coordinate is 0 or in [BOUNDED_TINY, BOUNDED_COORD] in magnitude,
                    // lo <= hi, every box holds its children's, and every leaf's triangles hold its box
-  uint32_t deep;   // 1 when a ray may come to hold more than QUAD_STACK entries: QuadWalker's GUARD
+                   // (2: and a ray may come to hold more than QUAD_STACK entries, QuadWalker's GUARD)
 };
 
 struct TraceHit {
@@ -594,7 +594,7 @@ struct QuadWalker {
   // A lane without a ray.
   __device__ __forceinline__ void idle() { ref = held = REF_NONE; }
 
-  // Ends the walk: the ray is walked again.
+  // Ends the walk (GUARD): the ray is walked again.
   __device__ __forceinline__ void hand_over() {
     hit.hit = RETRY;
     ref = held = REF_NONE;
@@ -604,7 +604,8 @@ struct QuadWalker {
   __device__ __forceinline__ bool aim(const SceneView& s, v3 o, v3 dir) {
     if (!(s.small != 0u && bounded_axis(o.x, dir.x) && bounded_axis(o.y, dir.y) && bounded_axis(o.z, dir.z) &&
           fabsf(dir.x) >= 1e-12f && fabsf(dir.y) >= 1e-12f && fabsf(dir.z) >= 1e-12f)) {
-      hand_over();
+      hit.hit = RETRY;
+      ref = REF_NONE;
       return false;
     }
     ox = pair(o.x, o.x);
