@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(THREADS, TRACE_WARPS_PER_SM * 32 / THREADS) k_
 // world or instance space), walked again from the start with IEEE division
 // throughout; its launch reads the count on the device, so a pass issues it
 // whether or not any ray needs it.
-template <bool ANY>
+template <bool ANY, bool FLAT>
 __global__ void __launch_bounds__(128) k_trace_queue_retry(const __grid_constant__ Pass P) {
   const uint32_t n = P.w.counters[ANY ? 14 : 13];
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(128) k_trace_queue_retry(const __grid_constant
     RefStack st;
     Walker<ANY, false, BOX_IEEE> w;
     w.start(P.s, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), ANY ? a.w : 1e20f);
-    w.run(P.s, st, [&](v3& o, v3& d) {
+    w.template run<FLAT>(P.s, st, [&](v3& o, v3& d) {
       o = mk3(a.x, a.y, a.z);
       d = mk3(b.x, b.y, b.z);
     });
@@ -1566,7 +1566,11 @@ void launch_trace_queue(int sel, uint32_t short_stack, const Pass& P, uint32_t w
   } else {
     launch_trace_queue_short<ANY, 0>(sel, P, which, st);
   }
-  k_trace_queue_retry<ANY><<<grids().retry * (P.s.small != 0u ? 1 : 8), 128, 0, st>>>(P);
+  const int retry = grids().retry * (P.s.small != 0u ? 1 : 8);
+  if (P.s.insts)
+    k_trace_queue_retry<ANY, false><<<retry, 128, 0, st>>>(P);
+  else
+    k_trace_queue_retry<ANY, true><<<retry, 128, 0, st>>>(P);
 }
 
 int thread_select(uint32_t threads) { return threads == 64u ? 0 : (threads == 256u ? 2 : 1); }

@@ -124,7 +124,7 @@ void trace_init(pfxt_trace& t, const pfxt_buffers& b, const pfxt_scene& view, co
   t.view.wide = t.d_wide;
   t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;
-  t.view.insts = t.d_insts;
+  t.view.insts = layout.insts.empty() ? nullptr : t.d_insts;
   t.view.root = layout.root;
   t.view.small = layout.small ? (layout.stack_need > QUAD_STACK ? 2u : 1u) : 0u;
   if (b.nodes_bytes >= sizeof(GpuNode)) {
@@ -384,7 +384,7 @@ void trace_move_scene(pfxt_trace& t, const pfxt_buffers& b, bool own) {
   t.view.wide = t.d_wide;
   t.view.quad = t.d_quad;
   t.view.tris = t.d_tris;
-  t.view.insts = t.d_insts;
+  t.view.insts = layout.insts.empty() ? nullptr : t.d_insts;
   t.view.root = layout.root;
   t.view.small = layout.small ? (layout.stack_need > QUAD_STACK ? 2u : 1u) : 0u;
   check(cudaMemcpy(t.d_surfaces, b.surfaces, b.surfaces_bytes, cudaMemcpyHostToDevice), "surfaces");
