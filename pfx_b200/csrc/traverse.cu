@@ -244,9 +244,10 @@ cudaError_t launch(const SceneView& s, const pfxt_ray* rays, uint32_t n, void* o
   const uint32_t lanes = lanes_per_warp(n, most * (kThreads / 32));
   const uint32_t blocks = std::min(most, (n + lanes * (kThreads / 32) - 1) / (lanes * (kThreads / 32)));
   k_trace<MODE, GUARD><<<blocks, kThreads, 0, stream>>>(s, rays, n, out, counter, lanes);
-  // a ray a thread where that is not too many blocks: a thread with several holds its
-  // warp up (2^21 rays of two axes in a room of 100k triangles: 767 -> 738 us)
-  const uint32_t scan = std::min(16u * most, (n + kThreads - 1) / kThreads);
+  // Few rays a thread, as a thread with several holds its warp up (2^21 rays of two axes
+  // in a room of 100k triangles, one batch of resident blocks and four: 767 and 740 us),
+  // but not one: 16 batches cost the scan of a batch without any 3 us at 1.5 M rays.
+  const uint32_t scan = std::min(4u * most, (n + kThreads - 1) / kThreads);
   if (s.insts)
     k_trace_retry<MODE, false><<<scan, kThreads, 0, stream>>>(s, rays, n, out);
   else
